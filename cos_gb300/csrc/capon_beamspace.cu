@@ -648,6 +648,417 @@ static int launch_tile(const FrameDev &f, float2 *R_out, cudaStream_t s)
     return cudaGetLastError();
 }
 
+// ---------------------------------------------------------------------------
+// Range-tile kernel for more beams (5 < Nb <= 32), Nb at run time.
+//
+// The warp kernel above redoes the DFT and the products of every window row
+// for every pixel and leaves the Nb x Nb solve to one lane; at M=64, L=32,
+// K=1, Nb=8 with weights it needs 3.90 ms for 65 k pixels, this kernel 0.26 ms
+// (13 GB/s -> 196 GB/s of the frame's own bytes).  Here a CTA owns a
+// run of pixels of one beam and does each row's work once:
+//   rows    Y[row][s][b] by the sliding DFT in chunks of kWideChunk subarrays
+//           (direct at the chunk start), the row's energy sum_m c_m |x_m|^2
+//           (c_m: how many subarrays hold channel m) and the beam sums;
+//   Q_row   the Nb x Nb products in 2 x 2 blocks per thread, four terms in
+//           FP32, chunk sums in float-float;
+//   window  R_bs per pixel, the float-float sum of its 2K+1 Q_row;
+//   solve   G lanes per pixel (8, 16 or 32 >= Nb), lane j holding column j of
+//           the upper triangle in registers, front-padded with an identity so
+//           that the unrolled steps below Nb are skipped: FP32 R = L D L^H with
+//           a_bs carried, back substitution, the residual a_bs - R x0 in
+//           float-float with exact high products, one correction.
+// What bounds it: issue of the FP32 pipe over short dependent loops; the tile
+// is the largest of 32, 16, 8 pixels that leaves two CTAs an SM to overlap
+// one's loads and barriers with the other's arithmetic.
+static constexpr int kWideThreads = 256;
+static constexpr int kWideChunk = 3;
+static constexpr int kWideMaxNb = 32;
+
+struct BsWideSmem {
+    int tile, rows, NbE, NQ;
+    size_t off_b, off_x, off_e, off_g, off_y, off_q, off_r, off_u, off_xb, total;
+    __host__ __device__ BsWideSmem(int tile_, int K, int M, int L, int Nb, int G)
+    {
+        tile = tile_;
+        rows = tile + 2 * K;
+        NbE = (Nb + 1) & ~1;
+        NQ = Nb * (Nb + 1) / 2;
+        const int Ns = M - L + 1;
+        auto up = [](size_t v) { return (v + 15) & ~(size_t)15; };
+        off_b = 0;                                                        // Butler L x NbE, rot, a_bs
+        off_x = off_b + up((size_t)(L * NbE + 2 * NbE) * sizeof(float2));
+        off_e = off_x + up((size_t)rows * M * sizeof(float2));
+        off_g = off_e + up((size_t)rows * sizeof(float));
+        off_q = off_g + up((size_t)rows * NbE * sizeof(float2));          // rows x NQ (hi, lo)
+        off_xb = off_q + up((size_t)rows * NQ * sizeof(float4));          // tile x (Nb + 1)
+        // Y is dead once the row products are formed: the pixels' matrices and
+        // the solve's exchange rows take its place
+        off_y = off_xb + up((size_t)tile * (Nb + 1) * sizeof(float2));
+        off_r = off_y;                                                    // tile x NQ (hi, lo)
+        off_u = off_r + up((size_t)tile * NQ * sizeof(float4));           // (256 / G) x G x (G + 1)
+        const size_t y_end = off_y + up((size_t)rows * Ns * NbE * sizeof(float2));
+        const size_t u_end = off_u + up((size_t)(kWideThreads / G) * G * (G + 1) * sizeof(float2));
+        total = y_end > u_end ? y_end : u_end;
+    }
+};
+
+// (h, l) += a x with a = (hi.re, hi.im, lo.re, lo.im): the high part's products
+// exact (TwoProd by fma), the low part's in FP32
+COS_DEV void bs_ff_cmac(float2 &h, float2 &l, float4 a, float2 x)
+{
+    const float2 xb = make_float2(-x.y, x.x);
+    const float2 sx = make_float2(a.x, a.x), sy = make_float2(a.y, a.y);
+    const float2 z = make_float2(0.f, 0.f);
+    const float2 p1 = ffma2(sx, x, z), p2 = ffma2(sy, xb, z);
+    const float2 e1 = ffma2(sx, x, make_float2(-p1.x, -p1.y)), e2 = ffma2(sy, xb, make_float2(-p2.x, -p2.y));
+    two_sum_acc(h, l, p1);
+    two_sum_acc(h, l, p2);
+    l = fadd2(l, fadd2(e1, e2));
+    l = ffma2(make_float2(a.z, a.z), x, l);
+    l = ffma2(make_float2(a.w, a.w), xb, l);
+}
+
+// i / d by the reciprocal of d; exact while the quotient times d stays below 2^21
+COS_DEV int bs_div(int i, float inv) { return (int)(((float)i + 0.5f) * inv); }
+
+template <int G>
+__global__ void __launch_bounds__(kWideThreads, 2)
+beamspace_wide_kernel(FrameDev f, float2 *__restrict__ Rbs, int tile, int units)
+{
+    extern __shared__ __align__(16) unsigned char smraw[];
+    __shared__ unsigned short blk[(kWideMaxNb / 2) * (kWideMaxNb / 2 + 1) / 2];
+    const int M = f.M, L = f.L, K = f.K, T = 2 * K + 1, Ns = M - L + 1, Nb = f.Nb;
+    const BsWideSmem S(tile, K, M, L, Nb, G);
+    const int NbE = S.NbE, NQ = S.NQ;
+    float2 *Bt = (float2 *)(smraw + S.off_b);   // [l][b]
+    float2 *rot = Bt + L * NbE, *ab = rot + NbE;
+    float2 *xs = (float2 *)(smraw + S.off_x);
+    float *Es = (float *)(smraw + S.off_e);
+    float2 *Gs = (float2 *)(smraw + S.off_g);
+    float2 *Y = (float2 *)(smraw + S.off_y);    // [row][s][b]
+    float4 *Qs = (float4 *)(smraw + S.off_q);
+    float4 *Rs = (float4 *)(smraw + S.off_r);
+    float2 *Xb = (float2 *)(smraw + S.off_xb);
+    const int tid = threadIdx.x;
+    const float isl = 1.0f / sqrtf((float)L);
+
+    // the Butler matrix, transposed; an odd Nb gets a zero beam beside the last
+    for (int i = tid; i < NbE * L; i += kWideThreads) {
+        const int l = i / NbE, bb = i % NbE;
+        float sn, cs;
+        sincospif(2.0f * (float)((butler_bin(bb, Nb, L) * l) % L) / (float)L, &sn, &cs);
+        Bt[i] = bb < Nb ? make_float2(cs * isl, -sn * isl) : make_float2(0.f, 0.f);
+    }
+    if (tid < NbE) {
+        float sn, cs;
+        sincospif(2.0f * (float)butler_bin(tid, Nb, L) / (float)L, &sn, &cs);
+        rot[tid] = make_float2(cs, sn);
+    }
+    __syncthreads();
+    // a_bs in float-float: it scales every output
+    if (tid < NbE) {
+        float2 hi = make_float2(0.f, 0.f), lo = hi;
+        for (int l = 0; l < L; ++l) two_sum_acc(hi, lo, Bt[l * NbE + tid]);
+        ab[tid] = fadd2(hi, lo);
+    }
+    // the 2 x 2 blocks of the upper triangle
+    const int nh = NbE / 2, nt = nh * (nh + 1) / 2;
+    for (int t = tid; t < nh * nh; t += kWideThreads) {
+        const int i = t / nh, j = t % nh;
+        if (i <= j) blk[i * nh - i * (i - 1) / 2 + (j - i)] = (unsigned short)((2 * i) << 8 | (2 * j));
+    }
+
+    const int tiles_per_beam = (f.Npy + tile - 1) / tile;
+#pragma unroll 1
+    for (int u = blockIdx.x; u < units; u += gridDim.x) {
+        const int bx = u / tiles_per_beam;
+        const int p0 = (u % tiles_per_beam) * tile;
+        const int np = min(tile, f.Npy - p0);
+        const int rows = np + 2 * K;
+        __syncthreads();   // the tables; the last tile's readers are done
+        const float2 *src = f.x + ((size_t)bx * f.Ny + p0) * M;
+        for (int i = tid; i < rows * M; i += kWideThreads) xs[i] = src[i];
+        __syncthreads();
+
+        // ---- rows: the sliding DFT, two beams per thread
+        {
+            const int nch = (Ns + kWideChunk - 1) / kWideChunk, nbp = NbE / 2;
+            const float inv_nbp = 1.f / (float)nbp, inv_nch = 1.f / (float)nch;
+            for (int it = tid; it < rows * nch * nbp; it += kWideThreads) {
+                const int rc = bs_div(it, inv_nbp), b = 2 * (it - rc * nbp), r = bs_div(rc, inv_nch), ch = rc - r * nch;
+                const int s0 = ch * kWideChunk, s1 = min(Ns, s0 + kWideChunk);
+                const float2 *xr = xs + (size_t)r * M;
+                float2 y0 = make_float2(0.f, 0.f), y1 = make_float2(0.f, 0.f);
+                for (int l = 0; l < L; ++l) {
+                    const float2 v = xr[s0 + l];
+                    const float4 bb = *(const float4 *)(Bt + l * NbE + b);
+                    y0 = cmac4(y0, make_float2(bb.x, bb.y), v);
+                    y1 = cmac4(y1, make_float2(bb.z, bb.w), v);
+                }
+                const float2 r0 = rot[b], r1 = rot[b + 1];
+                float2 *yr = Y + ((size_t)r * Ns + s0) * NbE + b;
+                *(float4 *)yr = make_float4(y0.x, y0.y, y1.x, y1.y);
+                for (int s = s0 + 1; s < s1; ++s) {
+                    yr += NbE;
+                    const float2 dx = cscale(csub(xr[s - 1 + L], xr[s - 1]), isl);
+                    y0 = cmul(r0, cadd(y0, dx));
+                    y1 = cmul(r1, cadd(y1, dx));
+                    *(float4 *)yr = make_float4(y0.x, y0.y, y1.x, y1.y);
+                }
+            }
+        }
+        // row energies sum_s sum_l |x[s+l]|^2, a warp per row
+        for (int r = tid >> 5; r < rows; r += kWideThreads / 32) {
+            float e = 0.f;
+            for (int m = tid & 31; m < M; m += 32)
+                e = fmaf((float)(min(min(m + 1, M - m), min(L, Ns))), cabs2(xs[(size_t)r * M + m]), e);
+            for (int o = 16; o; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+            if ((tid & 31) == 0) Es[r] = e;
+        }
+        __syncthreads();
+
+        // ---- Q_row, 2 x 2 beams per thread
+        {
+            const float inv_nt = 1.f / (float)nt, inv_nb = 1.f / (float)Nb;
+            for (int it = tid; it < rows * nt; it += kWideThreads) {
+                const int r = bs_div(it, inv_nt), e = blk[it - r * nt];
+                const int bi = e >> 8, bj = e & 255;
+                const float2 *y = Y + (size_t)r * Ns * NbE;
+                float2 hi[4], lo[4];
+    #pragma unroll
+                for (int q = 0; q < 4; ++q) hi[q] = lo[q] = make_float2(0.f, 0.f);
+                for (int s0 = 0; s0 < Ns; s0 += 4) {
+                    // u conj(v): P += (u.re, u.im).(v.re, v.im), Q += (u.im, -u.re).(v.re, v.im)
+                    float2 P[4], Q[4];
+    #pragma unroll
+                    for (int q = 0; q < 4; ++q) P[q] = Q[q] = make_float2(0.f, 0.f);
+    #pragma unroll
+                    for (int ss = 0; ss < 4; ++ss) {
+                        if (s0 + ss < Ns) {
+                            const float4 u = *(const float4 *)(y + (s0 + ss) * NbE + bi);
+                            const float4 v = *(const float4 *)(y + (s0 + ss) * NbE + bj);
+                            const float2 ur[2] = {make_float2(u.x, u.y), make_float2(u.z, u.w)};
+                            const float2 ui[2] = {make_float2(u.y, -u.x), make_float2(u.w, -u.z)};
+                            const float2 vv[2] = {make_float2(v.x, v.y), make_float2(v.z, v.w)};
+    #pragma unroll
+                            for (int q = 0; q < 4; ++q) {
+                                P[q] = ffma2(ur[q / 2], vv[q % 2], P[q]);
+                                Q[q] = ffma2(ui[q / 2], vv[q % 2], Q[q]);
+                            }
+                        }
+                    }
+    #pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        two_sum_acc(hi[q], lo[q], make_float2(P[q].x + P[q].y, Q[q].x + Q[q].y));
+                }
+    #pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int a = bi + q / 2, c = bj + q % 2;
+                    if (a <= c && c < Nb)
+                        Qs[(size_t)r * NQ + a * Nb - a * (a - 1) / 2 + (c - a)] =
+                            make_float4(hi[q].x, hi[q].y, lo[q].x, lo[q].y);
+                }
+            }
+            // beam sums of the row
+            for (int it = tid; it < rows * Nb; it += kWideThreads) {
+                const int r = bs_div(it, inv_nb), b = it - r * Nb;
+                float2 g0 = make_float2(0.f, 0.f), g1 = g0;
+                const float2 *y = Y + (size_t)r * Ns * NbE + b;
+                int s = 0;
+                for (; s + 1 < Ns; s += 2) {
+                    g0 = fadd2(g0, y[s * NbE]);
+                    g1 = fadd2(g1, y[(s + 1) * NbE]);
+                }
+                if (s < Ns) g0 = fadd2(g0, y[s * NbE]);
+                Gs[r * NbE + b] = fadd2(g0, g1);
+            }
+        }
+        __syncthreads();
+
+        // ---- window sums, renormalised: (value, remainder)
+        const float inv_nq = 1.f / (float)NQ;
+        for (int it = tid; it < np * NQ; it += kWideThreads) {
+            const int lp = bs_div(it, inv_nq), e = it - lp * NQ;
+            float2 h = make_float2(0.f, 0.f), l = h;
+            for (int t = 0; t < T; ++t) {
+                const float4 q = Qs[(size_t)(lp + t) * NQ + e];
+                two_sum_acc(h, l, make_float2(q.x, q.y));
+                l = fadd2(l, make_float2(q.z, q.w));
+            }
+            const float2 v = fadd2(h, l), w = fsub2(l, fsub2(v, h));
+            Rs[it] = make_float4(v.x, v.y, w.x, w.y);
+        }
+        __syncthreads();
+
+        // ---- solve, G lanes per pixel
+        {
+            const int g = tid / G, j = tid % G, pad = G - Nb, c = j - pad;   // lane j: column c of R_bs
+            float2 *X = (float2 *)(smraw + S.off_u) + (size_t)g * G * (G + 1);
+            auto idx = [&](int a, int b) { return a * Nb - a * (a - 1) / 2 + (b - a); };   // a <= b
+            const int per = kWideThreads / G;
+            for (int base = 0; base < np; base += per) {
+                const int lp = min(base + g, np - 1);   // a whole warp stays in step; the spare groups repeat a pixel
+                const bool own = base + g < np;
+                const float4 *R = Rs + (size_t)lp * NQ;
+                float dl;
+                if (f.loading == COS_CAPON_LOAD_ABSOLUTE) {
+                    dl = f.d * (float)(Ns * T);
+                } else if (f.loading == COS_CAPON_LOAD_BEAMSPACE) {
+                    float tb = 0.f;
+                    for (int i = 0; i < Nb; ++i) tb += R[idx(i, i)].x;
+                    dl = f.d * tb / (float)Nb;
+                } else {
+                    float tr = 0.f;
+                    for (int t = 0; t < T; ++t) tr += Es[lp + t];
+                    dl = f.d * tr / (float)L;
+                }
+                const long long pix = (long long)bx * f.Npy + p0 + lp;
+                float2 A[G];   // column j of D L^H, rows k <= j (padded index)
+    #pragma unroll
+                for (int k = 0; k < G; ++k) {
+                    A[k] = make_float2(0.f, 0.f);
+                    if (c >= 0 && k >= pad && k <= j) {
+                        const float4 v = R[idx(k - pad, c)];
+                        A[k] = k == j ? make_float2(v.x + dl, 0.f) : make_float2(v.x, v.y);
+                        if (Rbs && own) {   // loaded, unnormalised, column-major
+                            float2 *Rp = Rbs + (size_t)pix * Nb * Nb;
+                            Rp[(k - pad) + c * Nb] = A[k];
+                            if (k < j) Rp[c + (k - pad) * Nb] = cconj(A[k]);
+                        }
+                    }
+                }
+                const float2 a0 = c >= 0 ? ab[c] : make_float2(0.f, 0.f);
+                float2 y = a0;         // L^-1 a_bs, row j
+                float dinv = 1.f;      // 1 / d_j
+                // step i: row i of the factor in X[i], then the rows below
+                __syncwarp();
+    #pragma unroll
+                for (int i = 0; i < G; ++i) {
+                    if (i < pad) continue;   // the identity rows
+                    X[i * (G + 1) + j] = A[i];
+                    if (j == i) X[i * (G + 1) + G] = y;
+                    __syncwarp();
+                    const float rd = __frcp_rn(X[i * (G + 1) + i].x);
+                    const float2 yi = cscale(X[i * (G + 1) + G], rd);
+                    if (j == i) dinv = rd;
+                    if (j > i) {
+                        y = csub(y, cconjmul(A[i], yi));
+                        const float2 v = cscale(A[i], rd);
+    #pragma unroll
+                        for (int k = i + 1; k < G; ++k)   // rows k > j are never read
+                            A[k] = csub(A[k], cconjmul(X[i * (G + 1) + k], v));
+                    }
+                }
+                // back substitution D L^H x = y: row j of the factor lies in X[j]
+                auto back = [&](float2 v) {
+                    float2 x = make_float2(0.f, 0.f);
+                    for (int i = G - 1; i >= pad; --i) {
+                        const float2 xi = shfl2(cscale(v, dinv), i, G);
+                        if (j == i) x = xi;
+                        if (j < i && j >= pad) v = csub(v, cmul(X[j * (G + 1) + i], xi));
+                    }
+                    return x;
+                };
+                __syncwarp();
+                float2 x = back(y);
+                // residual a_bs - (R + dl I) x in float-float, row j
+                float2 h = make_float2(0.f, 0.f), lo = h;
+                for (int i = pad; i < G; ++i) {
+                    const float2 xi = shfl2(x, i, G);
+                    if (c >= 0) {
+                        float4 e = R[i >= j ? idx(c, i - pad) : idx(i - pad, c)];
+                        if (i < j) e = make_float4(e.x, -e.y, e.z, -e.w);
+                        if (i == j) e = make_float4(e.x, 0.f, e.z, 0.f);
+                        bs_ff_cmac(h, lo, e, xi);
+                    }
+                }
+                float2 r;
+                {
+                    const double rre = ((double)a0.x - (double)dl * (double)x.x) - (double)h.x - (double)lo.x;
+                    const double rim = ((double)a0.y - (double)dl * (double)x.y) - (double)h.y - (double)lo.y;
+                    r = make_float2((float)rre, (float)rim);
+                }
+                // forward solve with the column the lane holds
+    #pragma unroll
+                for (int i = 0; i < G; ++i) {
+                    if (i < pad) continue;
+                    const float2 ri = shfl2(cscale(r, dinv), i, G);
+                    if (j > i) r = csub(r, cconjmul(A[i], ri));
+                }
+                x = cadd(x, back(r));
+                // sum(Ria) = a_bs^H x; z = conj(x)^T g_bs / conj(sum), g_bs = beam sums / Ns
+                float2 aRa = make_float2(0.f, 0.f), zn = aRa;
+                if (c >= 0) {
+                    aRa = cconjmul(a0, x);
+                    zn = cconjmul(x, Gs[(lp + K) * NbE + c]);
+                }
+    #pragma unroll
+                for (int o = G / 2; o; o >>= 1) {
+                    aRa = cadd(aRa, shfl2_xor(aRa, o, G));
+                    zn = cadd(zn, shfl2_xor(zn, o, G));
+                }
+                const float den = cabs2(aRa);
+                const float2 isum = make_float2(aRa.x / den, -aRa.y / den);   // 1 / sum
+                if (own) {
+                    if (c >= 0) Xb[lp * (Nb + 1) + c] = x;
+                    if (j == 0) {
+                        Xb[lp * (Nb + 1) + Nb] = isum;
+                        if (f.z) f.z[pix] = cscale(cmul(zn, cconj(isum)), 1.0f / (float)Ns);
+                        if (f.P) f.P[pix] = 1.0f / ((float)Ns * (float)T * aRa.x);
+                    }
+                }
+            }
+        }
+        if (f.w) {
+            __syncthreads();
+            // w = B^H x_bs / sum, one thread per (pixel, element)
+            const float inv_l = 1.f / (float)L;
+            for (int i = tid; i < np * L; i += kWideThreads) {
+                const int lp = bs_div(i, inv_l), l = i - lp * L;
+                const float2 *xv = Xb + (size_t)lp * (Nb + 1), *bl = Bt + l * NbE;
+                float2 ria = make_float2(0.f, 0.f);
+                for (int b = 0; b < Nb; ++b) ria = cmac4_conj(ria, bl[b], xv[b]);
+                f.w[((size_t)bx * f.Npy + p0) * L + i] = cmul(ria, xv[Nb]);
+            }
+        }
+    }
+}
+
+// tile of the kernel above: two CTAs an SM where a tile of 8 pixels or more
+// allows it (smaller tiles for frames that would leave SMs idle), else the
+// largest that fits; 0 when none does
+static int wide_tile(const FrameDev &f, int G)
+{
+    for (int tile : {32, 16, 8})
+        if (BsWideSmem(tile, f.K, f.M, f.L, f.Nb, G).total <= 112 * 1024 &&
+            (tile == 8 || (long long)f.Nx * ((f.Npy + tile - 1) / tile) >= 152))
+            return tile;
+    for (int tile : {16, 8, 4, 2, 1})
+        if (BsWideSmem(tile, f.K, f.M, f.L, f.Nb, G).total <= 226 * 1024) return tile;
+    return 0;
+}
+
+template <int G>
+static int launch_wide(const FrameDev &f, float2 *R_out, int tile, cudaStream_t s)
+{
+    const BsWideSmem S(tile, f.K, f.M, f.L, f.Nb, G);
+    cudaError_t e = cudaFuncSetAttribute(beamspace_wide_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)S.total);
+    if (e != cudaSuccess) return e;
+    const long long units = (long long)f.Nx * ((f.Npy + tile - 1) / tile);
+    if (units > 0x7fffffffLL - 65536) return cudaErrorInvalidValue;
+    int dev = 0, sms = 0, per_sm = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
+        (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess ||
+        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, beamspace_wide_kernel<G>, kWideThreads, S.total)) !=
+            cudaSuccess)
+        return e;
+    // persistent CTAs: the tables are formed once each
+    const long long grid = units < (long long)sms * per_sm ? units : (long long)sms * per_sm;
+    beamspace_wide_kernel<G><<<(unsigned)grid, kWideThreads, S.total, s>>>(f, R_out, tile, (int)units);
+    return cudaGetLastError();
+}
+
 int launch_beamspace(const FrameDev &f, float2 *R_out, cudaStream_t s)
 {
     static_assert(kBeamspaceTileMaxNb == 5, "the tile kernel is instantiated for Nb = 1..5");
@@ -660,15 +1071,25 @@ int launch_beamspace(const FrameDev &f, float2 *R_out, cudaStream_t s)
     case 5: return launch_tile<5>(f, R_out, s);
     default: break;
     }
+    // the sizes served are the warp kernel's; within them the row-sharing
+    // kernel wherever a tile of it fits (3.90 -> 0.26 ms at M=64, L=32, K=1,
+    // Nb=8), Nb > 32 and very long windows with one warp per pixel
+    if (f.L > 64 || BsSmem(f.M, f.L, f.K, f.Nb).total > 227 * 1024) return cudaErrorNotSupported;
+    if (f.Nb <= kWideMaxNb) {
+        const int G = f.Nb <= 8 ? 8 : f.Nb <= 16 ? 16 : 32;
+        if (const int tile = wide_tile(f, G)) {
+            return G == 8    ? launch_wide<8>(f, R_out, tile, s)
+                   : G == 16 ? launch_wide<16>(f, R_out, tile, s)
+                             : launch_wide<32>(f, R_out, tile, s);
+        }
+    }
     return launch_beamspace_warp(f, R_out, s);
 }
 
 // one warp per pixel: any Nb <= L
 int launch_beamspace_warp(const FrameDev &f, float2 *R_out, cudaStream_t s)
 {
-    if (f.L > 64) return cudaErrorNotSupported;
     const BsSmem S(f.M, f.L, f.K, f.Nb);
-    if (S.total > 227 * 1024) return cudaErrorNotSupported;
     cudaError_t e = cudaFuncSetAttribute(beamspace_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)S.total);
     if (e != cudaSuccess) return e;
