@@ -264,6 +264,14 @@ static int run_plain(cos_capon_ctx *c, FrameDev f, cudaStream_t s)
     return e;
 }
 
+// general path for one element-space frame: covariance rows, then the register
+// solve
+static int run_general(cos_capon_ctx *c, FrameDev f, cudaStream_t s)
+{
+    if (int e = c->Rwork.ensure(general_bytes(f))) return e;
+    return launch_general(f, (float2 *)c->Rwork.p, c->d_status, c->num_sms, s);
+}
+
 // precise pipeline (float-float covariance, FP32 Cholesky, optional FP64-residual
 // refinement) for one element-space frame
 static int run_precise(cos_capon_ctx *c, FrameDev f, bool refine, cudaStream_t s)
@@ -409,10 +417,12 @@ static int run_frames(cos_capon_ctx *c, const FrameDev *fs, int n, const cos_cap
             }
             return e;
         }
-        // element space without a fused instantiation (or with refinement):
-        // the precise pipeline; the plain form when asked for
+        // element space without a fused instantiation: the general path where it
+        // serves the frame, else (refinement, few subarrays) the precise
+        // pipeline; the plain form when asked for
         return is_tc_form(o.form)                              ? run_tc(c, f, o.form, o.refine != 0, st)
                : (o.form == COS_CAPON_FORM_PLAIN && !o.refine) ? run_plain(c, f, st)
+               : general_supported(f)                          ? run_general(c, f, st)
                                                                : run_precise(c, f, o.refine != 0, st);
     };
     // Groups that use no context scratch (fused, beamspace) may run side by
@@ -588,6 +598,9 @@ static int get_capon_host(cos_capon_ctx *c, void *z, float *P, void *w, void *R,
     probe.M = M;
     probe.Nb = Nb;
     const bool plain = !use_fused(make_frame(probe, o), o);
+    cos_capon_frame whole = probe;
+    whole.Nx = Nx;
+    whole.Ny = Nz;
     size_t need = 0;
     need += bx > c->x.cap ? bx : 0;
     need += bz > c->z.cap ? bz : 0;
@@ -596,7 +609,8 @@ static int get_capon_host(cos_capon_ctx *c, void *z, float *P, void *w, void *R,
     need += (R && bR > c->R.cap) ? bR : 0;
     const bool sliding = o.form == COS_CAPON_FORM_SLIDING_INVERSE;
     if (plain && Nb == 0 && !sliding) {
-        need += (bR > c->Rwork.cap ? bR : 0) + (bw > c->Ria.cap ? bw : 0);
+        const size_t br = std::max(bR, general_bytes(make_frame(whole, o)));   // more than R at the shortest L
+        need += (br > c->Rwork.cap ? br : 0) + (bw > c->Ria.cap ? bw : 0);
         if (!(o.form == COS_CAPON_FORM_PLAIN && !o.refine)) need += bR > c->Rlo.cap ? bR : 0;
     }
     if ((e = check_free(need))) return e;

@@ -34,48 +34,12 @@
 #include "capon_common.cuh"
 #include "capon_fused_wide.cuh"
 #include "capon_internal.h"
+#include "capon_tma.cuh"
 #include "../../include/cos_capon.h"
 
 namespace cgb {
 namespace fused {
 
-// ---- mbarrier / bulk-copy primitives ---------------------------------------
-COS_DEV uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-COS_DEV void mbar_init(uint64_t *bar, uint32_t count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count));
-}
-COS_DEV void mbar_expect_tx(uint64_t *bar, uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes)
-                 : "memory");
-}
-COS_DEV bool mbar_try_wait(uint64_t *bar, uint32_t phase)
-{
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(smem_addr(bar)), "r"(phase)
-        : "memory");
-    return ok != 0;
-}
-// bounded wait; false when the limit was reached
-COS_DEV bool mbar_wait_bounded(uint64_t *bar, uint32_t phase, uint32_t limit = kWaitLimit)
-{
-    for (uint32_t it = 0; it < limit; ++it)
-        if (mbar_try_wait(bar, phase)) return true;
-    return false;
-}
-COS_DEV void bulk_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
-{
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smem_addr(dst)),
-        "l"(src), "r"(bytes), "r"(smem_addr(bar))
-        : "memory");
-}
 // timeout exit of thread 0: record it, then wait (bounded) for the bulk copies
 // still in flight into this CTA's shared memory -- buffer b (whose phase bit
 // was already flipped) and, when a next unit was issued, buffer b^1 -- so
@@ -95,9 +59,6 @@ static __device__ __noinline__ void stall_test_exit(unsigned *status, uint64_t *
     if (!mbar_wait_bounded(&bar[2], 0u, kStallTestLimit)) atomicOr(status, ERR_TIMEOUT);
     if (first_issued) mbar_wait_bounded(&bar[0], 0u);
 }
-COS_DEV void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-COS_DEV void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-
 // ---- compile-time configuration --------------------------------------------
 // L: subarray length; G: lanes per pixel (lane r owns columns j = m*G + r);
 // WARPS x NITER x (32/G) pixels per tile; T: the temporal window 2K+1 (exact,

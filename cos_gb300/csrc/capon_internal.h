@@ -60,6 +60,11 @@ int launch_plain_output(const FrameDev &f, const float2 *Ria, cudaStream_t s);
 // optional FP64-residual refinement); Rhi/Rlo hold Nx*Npy*L*L, dl Nx*Npy, Ria Nx*Npy*L
 int launch_precise(const FrameDev &f, float2 *Rhi, float2 *Rlo, float *dl, float2 *Ria, unsigned *status,
                    bool refine, cudaStream_t s);
+// general element-space path (any L, window, forward-backward averaging; no
+// refinement); work holds general_bytes
+bool general_supported(const FrameDev &f);
+size_t general_bytes(const FrameDev &f);
+int launch_general(const FrameDev &f, float2 *work, unsigned *status, int num_sms, cudaStream_t s);
 // FP32 Cholesky solve (optionally refined with an FP64 residual against
 // Rhi + Rlo + dl; Rlo may be null) and the output stage
 int launch_precise_solve(const FrameDev &f, const float2 *Rhi, const float2 *Rlo, const float *dl, float2 *Ria,
