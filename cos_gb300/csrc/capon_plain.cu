@@ -8,7 +8,6 @@
 //   * the covariance entry point cos_capon_build_r (IBuildR::getR),
 //   * the general path for subarray lengths the fused kernel does not
 //     instantiate.
-// The general LU solver for cos_capon_solve (ISolver::solve) is here too.
 #include <string.h>
 
 #include <mutex>
@@ -222,82 +221,6 @@ int launch_plain_output(const FrameDev &f, const float2 *Ria, cudaStream_t s)
     const long long npix = (long long)f.Nx * f.Npy;
     const long long blocks = (npix + kPlainWarps - 1) / kPlainWarps;
     plain_output_kernel<<<(unsigned)blocks, 32 * kPlainWarps, 0, s>>>(f, Ria);
-    return cudaGetLastError();
-}
-
-// ---------------------------------------------------------------------------
-// General batched solve A x = b (cos_capon_solve / ISolver::solve): one warp
-// per system, [A | b] in shared memory, Gaussian elimination with partial
-// pivoting by modulus, back substitution.  A column-major as in the
-// reference's Solver (testRTC.pyx:227-229 solves A^T x = b on row-major input).
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(32 * kPlainWarps)
-lu_solve_kernel(int N, long long batch, const float2 *__restrict__ Ag, const float2 *__restrict__ bg,
-                float2 *__restrict__ xg)
-{
-    extern __shared__ float2 smem[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long sys = (long long)blockIdx.x * kPlainWarps + warp;
-    if (sys >= batch) return;
-    const int ld = N + 2;  // columns 0..N-1 = A, column N = b
-    float2 *A = smem + (size_t)warp * N * ld;
-    const float2 *As = Ag + (size_t)sys * N * N;
-    for (int i = lane; i < N * N; i += 32) A[(i % N) * ld + i / N] = As[i];
-    for (int i = lane; i < N; i += 32) A[i * ld + N] = bg[(size_t)sys * N + i];
-    __syncwarp();
-    for (int i = 0; i < N; ++i) {
-        // pivot: row of max |A[r][i]| for r >= i
-        float best = -1.f;
-        int bi = i;
-        for (int r = i + lane; r < N; r += 32) {
-            const float v = cabs2(A[r * ld + i]);
-            if (v > best) { best = v; bi = r; }
-        }
-        for (int o = 16; o; o >>= 1) {
-            const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-        }
-        if (bi != i)
-            for (int c = lane; c <= N; c += 32) {
-                const float2 t = A[i * ld + c];
-                A[i * ld + c] = A[bi * ld + c];
-                A[bi * ld + c] = t;
-            }
-        __syncwarp();
-        const float2 piv = A[i * ld + i];
-        const float pd = cabs2(piv);
-        const float2 ipiv = make_float2(piv.x / pd, -piv.y / pd);
-        for (int r = i + 1; r < N; ++r) {
-            const float2 fct = cmul(A[r * ld + i], ipiv);
-            __syncwarp();
-            for (int c = i + 1 + lane; c <= N; c += 32)
-                A[r * ld + c] = csub(A[r * ld + c], cmul(fct, A[i * ld + c]));
-            __syncwarp();
-        }
-    }
-    if (lane == 0) {
-        for (int i = N - 1; i >= 0; --i) {
-            float2 v = A[i * ld + N];
-            for (int k = i + 1; k < N; ++k) v = csub(v, cmul(A[i * ld + k], A[k * ld + N + 1]));
-            const float2 piv = A[i * ld + i];
-            const float pd = cabs2(piv);
-            A[i * ld + N + 1] = cmul(v, make_float2(piv.x / pd, -piv.y / pd));
-        }
-    }
-    __syncwarp();
-    for (int i = lane; i < N; i += 32) xg[(size_t)sys * N + i] = A[i * ld + N + 1];
-}
-
-int launch_lu_solve(float2 *x, const float2 *A, const float2 *b, int N, int batch, cudaStream_t s)
-{
-    const size_t smem = (size_t)kPlainWarps * N * (N + 2) * sizeof(float2);
-    if (smem > 227 * 1024) return cudaErrorLaunchFailure;
-    cudaError_t e = cudaFuncSetAttribute(lu_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return e;
-    const long long blocks = ((long long)batch + kPlainWarps - 1) / kPlainWarps;
-    lu_solve_kernel<<<(unsigned)blocks, 32 * kPlainWarps, smem, s>>>(N, batch, A, b, x);
     return cudaGetLastError();
 }
 
