@@ -8,77 +8,112 @@
 //       s_w = sum_{yy,xx} |Z[y+yy-Ymid][x+xx-Xmid][w]|^2 wrf[yy][xx],
 //     the first w of least s_w is selected; img = Z[y][x][w*], win = w*;
 //     border pixels keep img = 0, win = 0.
-// Two passes: |Z|^2 into planes [Nw][Ny][Nx] (coalesced along x), then one
-// thread per pixel forms the Nw weighted sums (FP32) and the argmin.
+//
+// One pass: a CTA brings its tile of Z, with the filter's halo, through |.|^2
+// into shared memory, up to W = 4 or 8 windows a pixel at a time (more go in
+// chunks, the best so far in registers), and a thread per pixel carries the W
+// sums through the filter (FP32, yy then xx), a tap being one weight and one or
+// two 16-byte loads for all W windows.  What bounds it: issue, about 15
+// instructions a tap, then the read of Z; a [2048][256] image with 8 windows and a
+// 5 x 1 filter takes 18 us (2.2 TB/s over Z once and the outputs).  As two passes
+// over memory, the planes |Z|^2 in HBM between them, it took 60 us; with a scalar
+// load, a multiply-add and the index arithmetic for every tap and window, 55 us.
+#include <algorithm>
+
 #include "capon_common.cuh"
 #include "capon_internal.h"
 #include "../../include/cos_capon.h"
 
 namespace cgb {
 
-__global__ void lca_power_kernel(const float2 *__restrict__ Z, int Ny, int Nx, int Nw, float *__restrict__ pw)
-{
-    const long long n = (long long)Ny * Nx * Nw;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int w = (int)(i % Nw);
-        const long long pix = i / Nw;   // y * Nx + x
-        pw[(long long)w * Ny * Nx + pix] = cabs2(Z[i]);
-    }
-}
+static constexpr int kLcaTX = 32, kLcaTY = 16, kLcaThreads = 512;
 
-__global__ void lca_select_kernel(LcaDev a)
+// W: windows a pixel holds in shared memory, S: its stride there in floats (8
+// lanes of a 16-byte load fall on all 32 banks: 4 and 12)
+template <int W>
+__global__ void __launch_bounds__(kLcaThreads, 2) lca_kernel(LcaDev a)
 {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-    if (x >= a.Nx || y >= a.Ny) return;
-    const long long pix = (long long)y * a.Nx + x;
-    const long long plane = (long long)a.Ny * a.Nx;
+    constexpr int S = W == 4 ? 4 : 12;
+    extern __shared__ __align__(16) float pw[];
+    const int x0 = blockIdx.x * kLcaTX, y0 = blockIdx.y * kLcaTY;
+    const int cols = kLcaTX + a.Xf - 1, rows = kLcaTY + a.Yf - 1;
+    const int tid = threadIdx.x, tx = tid % kLcaTX, ty = tid / kLcaTX, x = x0 + tx, y = y0 + ty;
+    const bool in = x < a.Nx && y < a.Ny;
+    // a 1 x 1 filter has no border: Ymid = Xmid = 0
+    const bool inner = in && y >= a.Ymid && y < a.Ny - a.Ymid && x >= a.Xmid && x < a.Nx - a.Xmid;
+    const float inv = 1.f / (float)cols;
     int best = 0;
-    if (a.single) {
-        float bv = 0.f;
-        for (int w = 0; w < a.Nw; ++w) {
-            const float v = a.pw[w * plane + pix];
-            if (w == 0 || v < bv) {
-                bv = v;
-                best = w;
-            }
+    float bv = 0.f;
+    for (int w0 = 0; w0 < a.Nw; w0 += W) {
+        const int nw = min(W, a.Nw - w0);
+        if (w0) __syncthreads();  // the last chunk's readers are done
+#pragma unroll 5
+        for (int i = tid; i < rows * cols * W; i += kLcaThreads) {
+            const int px = i / W, w = i % W;
+            // px / cols by the reciprocal: exact below 2^21
+            const int r = (int)(((float)px + 0.5f) * inv);
+            const int yy = y0 - a.Ymid + r, xx = x0 - a.Xmid + px - r * cols;
+            float v = 0.f;
+            if (w < nw && yy >= 0 && yy < a.Ny && xx >= 0 && xx < a.Nx)
+                v = cabs2(a.Z[((long long)yy * a.Nx + xx) * a.Nw + (w0 + w)]);
+            pw[px * S + w] = v;
         }
-    } else {
-        if (y < a.Ymid || y >= a.Ny - a.Ymid || x < a.Xmid || x >= a.Nx - a.Xmid) {
-            a.img[pix] = make_float2(0.f, 0.f);
-            if (a.win) a.win[pix] = 0;
-            return;
-        }
-        float bv = 0.f;
-        for (int w = 0; w < a.Nw; ++w) {
-            const float *p = a.pw + w * plane;
-            float s = 0.f;
-            for (int yy = 0; yy < a.Yf; ++yy) {
-                const float *row = p + (long long)(y + yy - a.Ymid) * a.Nx + (x - a.Xmid);
-                for (int xx = 0; xx < a.Xf; ++xx) s = fmaf(row[xx], a.wrf[yy * a.Xf + xx], s);
+        __syncthreads();
+        if (inner) {
+            float s[W];
+#pragma unroll
+            for (int w = 0; w < W; ++w) s[w] = 0.f;
+            const float *p = pw + (ty * cols + tx) * S;
+            if (a.single) {
+#pragma unroll
+                for (int w = 0; w < W; ++w) s[w] = p[w];
+            } else {
+                for (int yy = 0, k = 0; yy < a.Yf; ++yy, p += (cols - a.Xf) * S)
+#pragma unroll 1
+                    for (int xx = 0; xx < a.Xf; ++xx, ++k, p += S) {
+                        const float wgt = a.wrf[k];
+#pragma unroll
+                        for (int q = 0; q < W / 4; ++q) {
+                            const float4 v = ((const float4 *)p)[q];
+                            s[4 * q] = fmaf(v.x, wgt, s[4 * q]);
+                            s[4 * q + 1] = fmaf(v.y, wgt, s[4 * q + 1]);
+                            s[4 * q + 2] = fmaf(v.z, wgt, s[4 * q + 2]);
+                            s[4 * q + 3] = fmaf(v.w, wgt, s[4 * q + 3]);
+                        }
+                    }
             }
-            if (w == 0 || s < bv) {
-                bv = s;
-                best = w;
-            }
+#pragma unroll
+            for (int w = 0; w < W; ++w)
+                if (w < nw && (w0 + w == 0 || s[w] < bv)) {
+                    bv = s[w];
+                    best = w0 + w;
+                }
         }
     }
-    a.img[pix] = a.Z[pix * a.Nw + best];
-    if (a.win) a.win[pix] = best;
+    if (in) {
+        const long long pix = (long long)y * a.Nx + x;
+        a.img[pix] = inner ? a.Z[pix * a.Nw + best] : make_float2(0.f, 0.f);
+        if (a.win) a.win[pix] = best;
+    }
 }
 
-int launch_lca(const LcaDev &a, float *pw, cudaStream_t s)
+template <int W>
+static int launch_w(const LcaDev &a, cudaStream_t s)
 {
-    const long long n = (long long)a.Ny * a.Nx * a.Nw;
-    long long blocks = (n + 255) / 256;
-    if (blocks > 152 * 32) blocks = 152 * 32;
-    lca_power_kernel<<<(unsigned)blocks, 256, 0, s>>>(a.Z, a.Ny, a.Nx, a.Nw, pw);
-    cudaError_t e = cudaGetLastError();
+    const size_t smem = (size_t)(kLcaTX + a.Xf - 1) * (kLcaTY + a.Yf - 1) * (W == 4 ? 4 : 12) * sizeof(float);
+    cudaError_t e = cudaFuncSetAttribute(lca_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    LcaDev b = a;
-    b.pw = pw;
-    dim3 grid((unsigned)((a.Nx + 127) / 128), (unsigned)a.Ny);
-    lca_select_kernel<<<grid, 128, 0, s>>>(b);
+    const dim3 grid((unsigned)((a.Nx + kLcaTX - 1) / kLcaTX), (unsigned)((a.Ny + kLcaTY - 1) / kLcaTY));
+    lca_kernel<W><<<grid, kLcaThreads, smem, s>>>(a);
     return cudaGetLastError();
+}
+
+int launch_lca(const LcaDev &a, cudaStream_t s)
+{
+    // W = 4 for few windows, and where the halo of a long filter (up to 256 taps)
+    // leaves no room for 8: at most 32 x 271 pixels of 16 bytes, 139 KB
+    const size_t n = (size_t)(kLcaTX + a.Xf - 1) * (kLcaTY + a.Yf - 1);
+    return a.Nw <= 4 || n * 12 * sizeof(float) > 112 * 1024 ? launch_w<4>(a, s) : launch_w<8>(a, s);
 }
 
 }  // namespace cgb

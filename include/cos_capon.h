@@ -127,7 +127,7 @@ typedef struct cos_capon_ctx cos_capon_ctx;
  * device status word -- the role of the reference's Capon object
  * (Capon.h:13-125, Capon.cpp:50-71).  Uses the calling thread's current device.
  * Like that object, a context is not thread-safe: its work buffers (the
- * materialised-R pipelines, the LCA planes, the staging of host calls) serve
+ * materialised-R pipelines, the staging of host calls) serve
  * one call at a time, so calls that may overlap -- from several threads, or
  * device calls on different streams -- need a context each. */
 int cos_capon_create(cos_capon_ctx **ctx);
