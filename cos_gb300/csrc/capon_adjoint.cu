@@ -13,8 +13,8 @@
 // Only the saved weights are needed: the covariance's adjoint is applied in
 // factored form through e_ts, so R is neither stored nor rebuilt.
 //
-// Work units are range tiles of one beam (as in the forward kernel).  The CTA
-// stages the tile's TILE+2K rows, each warp takes pixels of the tile, and the
+// The general kernel's work units are range tiles of one beam (as in the forward
+// kernel).  The CTA stages the tile's TILE+2K rows, each warp takes pixels of the tile, and the
 // gradient rows are accumulated in shared memory; rows only this tile touches
 // are added to the output directly, the 2K rows at each end (shared with the
 // neighbouring tiles) with atomics.  Tiles without incoming gradient are
@@ -123,158 +123,246 @@ __global__ void __launch_bounds__(32 * kAdjWarps) adjoint_kernel(AdjDev a)
     if (a.gd && lane == 0 && dacc != 0.f) atomicAdd(a.gd, dacc);
 }
 
-// Blocks of the register-blocked kernel and its shared-memory row padding:
-// odd block lengths and an odd row pad spread the lanes of one load over the
-// banks (at M=64, L=32, K=2 at most 2-3 lanes share a bank pair).
-static constexpr int kAdjSB = 7, kAdjCB = 11, kAdjPad = 3;
+// The same adjoint by range rows, for L = 8, 16, 24, 32.  A pair (pixel p, window
+// row t) adds to row y = p + t only, so a warp owns a row and gathers from the T
+// pixels whose window holds it: every pair is formed once, a gradient row is
+// complete in its warp, and neither the tile's rows nor the 2K rows between tiles
+// need atomics (the tile form above adds every pair into shared memory with
+// them).
+//
+// A lane takes (t, SB consecutive subarrays s) and holds the pixel's L weights in
+// registers for both products:
+//   e_s = w^H x[s .. s+L-1]      each sample meets w_l for every (s, l) with
+//                                s - s0 + l = i: two packed fmas, real and
+//                                imaginary part each as a sum over the pair
+//                                (w.re, w.im);
+//   G[c] += sum_s e_s w_{c-s}    with the same e_s still in registers, over the
+//                                SB + L - 1 channels they reach, added to the
+//                                row's accumulator of window row t in shared
+//                                memory.  At one step the lanes of a t write
+//                                different channels, and a warp barrier orders
+//                                the steps.  (Gathered by channel, half the
+//                                products are with s outside 0 .. Ns-1.)
+// The next row's samples and weights arrive by cp.async under this row's products
+// (398 -> 335 us together with the gradient rows leaving as vector reductions
+// instead of a load and a store).  What bounds it: the FP32 pipe over the useful
+// lanes (30 of 32 at M=64, L=32, K=2), issue 58 %.  Gradients at [128][1024][64],
+// L=32, K=2: 335 us, 625 us as tiles.
+static constexpr int kRowWarps = 8;
 
-// The same adjoint with the weights held in registers (L a template
-// parameter) and both products register-blocked, for L = 8, 16, 32:
-//   e_ts for SB consecutive s of one row t per lane: each sample x_t[s0+i]
-//        is loaded once and meets w_l for every (s, l) with s - s0 + l = i;
-//   G_t[c] = sum_s e_ts w_{c-s} for CB consecutive channels per lane: each
-//        e_ts is loaded once and meets w_l for every (c, l) with c - l = s.
-// Loads per complex multiply-add fall from two (the kernel above, bound by
-// shared-memory bandwidth) to (SB + L - 1) / (SB L) and (CB + L - 1) / (CB L).
-template <int LT>
-__global__ void __launch_bounds__(32 * kAdjWarps) adjoint_blocked_kernel(AdjDev a)
+struct AdjRowSmem {
+    int xs, ws, as;        // strides: samples, weights, accumulators
+    size_t off_w, off_a, per_warp, total;
+    __host__ __device__ AdjRowSmem(int M, int L, int T, int SB)
+    {
+        // strides that keep the 16-byte accesses of eight lanes on different
+        // banks: of the T pixels' weights, and of the accumulators at SB = 6
+        xs = (M + SB + 3) & ~1;      // zero tail: the last block's samples past the row
+        ws = L + 2;
+        as = ((M + SB - 4 + 15) & ~15) + 4;
+        // samples and weights twice: the next row's arrive during this row's products
+        off_w = (size_t)2 * xs * sizeof(float2);
+        off_a = off_w + (size_t)2 * (T + 1) * ws * sizeof(float2);   // T + 1: lanes without an item
+        per_warp = (off_a + (size_t)(T + 1) * as * sizeof(float2) + 15) & ~(size_t)15;
+        total = kRowWarps * per_warp + (size_t)kRowWarps * M * sizeof(float);
+    }
+};
+
+// 8 bytes global to shared, zeros when !is
+COS_DEV void async_copy8(void *dst, const void *src, bool is)
 {
-    constexpr int SB = kAdjSB, CB = kAdjCB;
-    extern __shared__ float2 smem[];
-    const int M = a.M, K = a.K, T = 2 * K + 1, Ns = M - LT + 1, XS = M + kAdjPad;
-    const int rows = kAdjTile + 2 * K;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    float2 *xs = smem;                          // rows x XS
-    float2 *gs = xs + (size_t)rows * XS;        // rows x XS gradient accumulator
-    float *ths = (float *)(gs + (size_t)rows * XS);  // M channel sums
-    float2 *wbuf = (float2 *)(ths + ((M + 1) & ~1)) + (size_t)warp * (LT + T * Ns);
-    float2 *ws = wbuf, *es = wbuf + LT;
-    const float scale = 1.0f / ((float)Ns * (float)T);
-    const int tiles_per_beam = (a.Npy + kAdjTile - 1) / kAdjTile;
-    const long long units = (long long)a.Nx * tiles_per_beam;
-    const int nsb = (Ns + SB - 1) / SB, ncb = (M + CB - 1) / CB;
-    float dacc = 0.f;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+                 "r"(is ? 8 : 0)
+                 : "memory");
+}
 
-    for (int i = tid; i < M; i += blockDim.x) ths[i] = 0.f;
-    for (long long u = blockIdx.x; u < units; u += gridDim.x) {
-        const int bx = (int)(u / tiles_per_beam);
-        const int p0 = (int)(u % tiles_per_beam) * kAdjTile;
-        const int np = min(kAdjTile, a.Npy - p0);
-        const int nr = np + 2 * K;
-        bool any = false;
-        for (int q = lane; q < np; q += 32) any |= (a.gP[(size_t)bx * a.Npy + p0 + q] != 0.f);
-        if (!__syncthreads_or(any)) continue;
-        const float2 *xg = a.x + ((size_t)bx * a.Ny + p0) * M;
-        for (int i = tid; i < nr * M; i += blockDim.x) {
-            const int r = i / M, c = i % M;
-            xs[r * XS + c] = xg[i];
-            gs[r * XS + c] = make_float2(0.f, 0.f);
+template <int L, int SB>
+__global__ void __launch_bounds__(32 * kRowWarps, 2) adjoint_row_kernel(AdjDev a)
+{
+    static_assert(SB % 2 == 0 && L % 2 == 0, "channel pairs are 16 bytes");
+    extern __shared__ __align__(16) unsigned char smraw[];
+    const int M = a.M, T = 2 * a.K + 1, Ns = M - L + 1;
+    const AdjRowSmem S(M, L, T, SB);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    unsigned char *const mine = smraw + warp * S.per_warp;
+    float2 *const acc = (float2 *)(mine + S.off_a);
+    float *const ths = (float *)(smraw + kRowWarps * S.per_warp) + (size_t)warp * M;   // channel-phase sums
+    const float scale = 1.0f / ((float)Ns * (float)T);
+    const int nsb = (Ns + SB - 1) / SB, items = T * nsb;
+    float dacc = 0.f;
+    for (int c = lane; c < M; c += 32) ths[c] = 0.f;
+    for (int b = 0; b < 2; ++b) {   // the zero tails: samples past M, weights of the lanes without an item
+        for (int c = M + lane; c < S.xs; c += 32) ((float2 *)mine)[b * S.xs + c] = make_float2(0.f, 0.f);
+        for (int l = lane; l < L; l += 32)
+            ((float2 *)(mine + S.off_w))[(b * (T + 1) + T) * S.ws + l] = make_float2(0.f, 0.f);
+    }
+    const long long rows = (long long)a.Nx * a.Ny, step = (long long)gridDim.x * kRowWarps;
+    // gradient of pixel y-t on lane t (T <= 32); 0 where there is none
+    auto grad = [&](long long row) {
+        const int bx = (int)(row / a.Ny), p = (int)(row % a.Ny) - lane;
+        return row < rows && lane < T && p >= 0 && p < a.Npy ? a.gP[(size_t)bx * a.Npy + p] : 0.f;
+    };
+    // the row's samples and the weights of its pixels (zeros where there is none)
+    // into buffer b
+    auto stage = [&](long long row, int b) {
+        const int bx = (int)(row / a.Ny), y = (int)(row % a.Ny);
+        float2 *const xd = (float2 *)mine + b * S.xs, *const wd = (float2 *)(mine + S.off_w) + b * (T + 1) * S.ws;
+        const float2 *xr = a.x + (size_t)row * M;
+        for (int c = lane; c < M; c += 32) async_copy8(xd + c, xr + c, true);
+        for (int i = lane; i < T * L; i += 32) {
+            const int t = i / L, l = i % L, p = y - t;
+            const bool is = p >= 0 && p < a.Npy;
+            async_copy8(wd + t * S.ws + l, a.w + ((size_t)bx * a.Npy + (is ? p : 0)) * L + l, is);
         }
-        __syncthreads();
-        for (int q = warp; q < np; q += kAdjWarps) {
-            const long long pix = (long long)bx * a.Npy + p0 + q;
-            const float g = a.gP[pix];
-            if (g == 0.f) continue;  // warp-uniform
-            for (int l = lane; l < LT; l += 32) ws[l] = a.w[(size_t)pix * LT + l];
-            __syncwarp();
-            float2 wr[LT];
-            float wn = 0.f;
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    long long row = (long long)blockIdx.x * kRowWarps + warp;
+    float gnext = grad(row);
+    if (row < rows) stage(row, 0);
+    int b = 0;
+    for (; row < rows; row += step, b ^= 1) {
+        const float gl = gnext;
+        gnext = grad(row + step);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncwarp();   // the row has arrived for every lane, and the last one's readers are done
+        if (row + step < rows) stage(row + step, b ^ 1);
+        const float2 *const xw = (const float2 *)mine + b * S.xs;
+        float2 *const ws = (float2 *)(mine + S.off_w) + b * (T + 1) * S.ws;
+        // a pixel without a gradient takes no part, its weights finite or not; a row
+        // of such pixels gets nothing
+        const unsigned on = __ballot_sync(0xffffffffu, gl != 0.f);
+        if (on == 0u) continue;
+        for (int t = 0; t < T; ++t)
+            if (!(on >> t & 1u))
+                for (int l = lane; l < L; l += 32) ws[t * S.ws + l] = make_float2(0.f, 0.f);
+        for (int i = lane; i < (T + 1) * S.as; i += 32) acc[i] = make_float2(0.f, 0.f);
+        __syncwarp();
+        for (int it0 = 0; it0 < items; it0 += 32) {
+            const int it = it0 + lane, t = it < items ? it / nsb : T, s0 = it < items ? (it - t * nsb) * SB : 0;
+            const float gt = __shfl_sync(0xffffffffu, gl, t < T ? t : 0), g = t < T ? gt : 0.f;
+            float2 w[L];
 #pragma unroll
-            for (int l = 0; l < LT; ++l) {
-                wr[l] = ws[l];
-                wn += cabs2(wr[l]);
+            for (int l = 0; l < L; l += 2) {
+                const float4 v = *(const float4 *)(ws + t * S.ws + l);
+                w[l] = make_float2(v.x, v.y);
+                w[l + 1] = make_float2(v.z, v.w);
             }
-            if (lane == 0) dacc += g * wn;
-            // e_ts = w^H x_ts
-            for (int it = lane; it < T * nsb; it += 32) {
-                const int t = it / nsb, s0 = (it % nsb) * SB;
-                const float2 *xt = xs + (size_t)(q + t) * XS;
-                float2 acc[SB];
+            if (it < nsb) {   // t = 0: pixel y; one lane adds g |w|^2
+                float wn = 0.f;
 #pragma unroll
-                for (int j = 0; j < SB; ++j) acc[j] = make_float2(0.f, 0.f);
+                for (int l = 0; l < L; ++l) wn += cabs2(w[l]);
+                if (it == 0) dacc += g * wn;
+            }
+            // e_s, s = s0 .. s0+SB-1: (re, im) parts as pair sums
+            float2 er[SB], ei[SB];
 #pragma unroll
-                for (int i = 0; i < SB + LT - 1; ++i) {
-                    const float2 v = xt[min(s0 + i, M - 1)];  // past the row only for s >= Ns (not stored)
+            for (int j = 0; j < SB; ++j) er[j] = ei[j] = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < SB + L - 1; i += 2) {
+                const float4 q = *(const float4 *)(xw + s0 + i);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const float2 v = h ? make_float2(q.z, q.w) : make_float2(q.x, q.y);
+                    const float2 u = make_float2(v.y, -v.x);
 #pragma unroll
                     for (int j = 0; j < SB; ++j) {
-                        const int l = i - j;
-                        if (l >= 0 && l < LT) acc[j] = cmac4_conj(acc[j], wr[l], v);
-                    }
-                }
-#pragma unroll
-                for (int j = 0; j < SB; ++j)
-                    if (s0 + j < Ns) es[t * Ns + s0 + j] = acc[j];
-            }
-            __syncwarp();
-            // dP/dconj(x_t[c]) = scale g sum_s e_ts w_{c-s} into the shared accumulator
-            const float gsc = g * scale;
-            for (int it = lane; it < T * ncb; it += 32) {
-                const int t = it / ncb, c0 = (it % ncb) * CB;
-                const float2 *et = es + t * Ns;
-                float2 G[CB];
-#pragma unroll
-                for (int b = 0; b < CB; ++b) G[b] = make_float2(0.f, 0.f);
-#pragma unroll
-                for (int i = 0; i < LT + CB - 1; ++i) {
-                    const int sidx = c0 - (LT - 1) + i;
-                    const bool in = sidx >= 0 && sidx < Ns;
-                    const float2 ev = et[min(max(sidx, 0), Ns - 1)];
-                    const float2 e = make_float2(in ? ev.x : 0.f, in ? ev.y : 0.f);
-#pragma unroll
-                    for (int b = 0; b < CB; ++b) {
-                        const int l = b + LT - 1 - i;
-                        if (l >= 0 && l < LT) G[b] = cmac4(G[b], e, wr[l]);
-                    }
-                }
-                float2 *dst = gs + (size_t)(q + t) * XS + c0;
-#pragma unroll
-                for (int b = 0; b < CB; ++b) {
-                    if (c0 + b < M) {
-                        atomicAdd(&dst[b].x, G[b].x * gsc);
-                        atomicAdd(&dst[b].y, G[b].y * gsc);
+                        const int l = i + h - j;
+                        if (l >= 0 && l < L) {
+                            // conj(w) v = (w.re v.re + w.im v.im, w.re v.im - w.im v.re)
+                            er[j] = ffma2(w[l], v, er[j]);
+                            ei[j] = ffma2(w[l], u, ei[j]);
+                        }
                     }
                 }
             }
-            __syncwarp();
-        }
-        __syncthreads();
-        // write the tile's gradient rows; the channel-phase sums use them
-        float2 *gout = a.gx + ((size_t)bx * a.Ny + p0) * M;
-        for (int i = tid; i < nr * M; i += blockDim.x) {
-            const int r = i / M, c = i % M;
-            const float2 G = gs[r * XS + c];
-            if (G.x == 0.f && G.y == 0.f) continue;
-            const float2 xv = xs[r * XS + c];
-            atomicAdd(&ths[c], 2.f * (G.x * xv.y - G.y * xv.x));
-            if (r < 2 * K || r >= np) {
-                atomicAdd(&gout[i].x, G.x);
-                atomicAdd(&gout[i].y, G.y);
-            } else {
-                const float2 o = gout[i];
-                gout[i] = make_float2(o.x + G.x, o.y + G.y);
+            // e_s g / (Ns T) as (re, -im) and (im, re)
+            const float gs = g * scale;
+#pragma unroll
+            for (int j = 0; j < SB; ++j) {
+                const bool in = s0 + j < Ns;
+                const float re = in ? (er[j].x + er[j].y) * gs : 0.f, im = in ? (ei[j].x + ei[j].y) * gs : 0.f;
+                er[j] = make_float2(re, -im);
+                ei[j] = make_float2(im, re);
+            }
+            float2 *const at = acc + t * S.as + s0;
+#pragma unroll
+            for (int i = 0; i < SB + L - 1; i += 2) {
+                float2 G[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    float2 pr = make_float2(0.f, 0.f), pi = pr;
+#pragma unroll
+                    for (int j = 0; j < SB; ++j) {
+                        const int l = i + h - j;
+                        if (l >= 0 && l < L) {
+                            pr = ffma2(er[j], w[l], pr);
+                            pi = ffma2(ei[j], w[l], pi);
+                        }
+                    }
+                    G[h] = make_float2(pr.x + pr.y, pi.x + pi.y);
+                }
+                float4 *const d = (float4 *)(at + i);
+                const float4 o = *d;
+                *d = make_float4(o.x + G[0].x, o.y + G[0].y, o.z + G[1].x, o.w + G[1].y);
+                __syncwarp();
             }
         }
-        __syncthreads();
+        // the row's gradient, and its share of the channel phases
+        float2 *gout = a.gx + (size_t)row * M;
+        for (int c = lane; c < M; c += 32) {
+            float2 G = acc[c];
+            for (int t = 1; t < T; ++t) G = cadd(G, acc[t * S.as + c]);
+            const float2 xv = xw[c];
+            ths[c] += 2.f * (G.x * xv.y - G.y * xv.x);
+            // added without waiting for the old value
+            asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(gout + c), "f"(G.x), "f"(G.y) : "memory");
+        }
     }
-    if (a.gth)
-        for (int i = tid; i < M; i += blockDim.x)
-            if (ths[i] != 0.f) atomicAdd(&a.gth[i], ths[i]);
     if (a.gd && lane == 0 && dacc != 0.f) atomicAdd(a.gd, dacc);
+    __syncthreads();
+    if (a.gth) {
+        const float *all = (const float *)(smraw + kRowWarps * S.per_warp);
+        for (int c = threadIdx.x; c < M; c += blockDim.x) {
+            float v = 0.f;
+            for (int k = 0; k < kRowWarps; ++k) v += all[(size_t)k * M + c];
+            if (v != 0.f) atomicAdd(&a.gth[c], v);
+        }
+    }
 }
 
 template <class Kern>
-static int launch_adjoint_with(Kern kern, const AdjDev &a, size_t smem, int num_sms, cudaStream_t s)
+static int launch_adjoint_with(Kern kern, const AdjDev &a, long long units, size_t smem, int num_sms, cudaStream_t s)
 {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kAdjWarps, smem);
     if (e != cudaSuccess) return e;
-    const long long units = (long long)a.Nx * ((a.Npy + kAdjTile - 1) / kAdjTile);
     long long grid = (long long)num_sms * (per_sm > 0 ? per_sm : 1);
     if (grid > units) grid = units;
     kern<<<(unsigned)grid, 32 * kAdjWarps, smem, s>>>(a);
     return cudaGetLastError();
+}
+
+// SB: the block length that keeps the lanes fullest, passes of 32 items by the
+// products of an item
+template <int L>
+static int launch_rows(const AdjDev &a, int num_sms, cudaStream_t s)
+{
+    static_assert(kRowWarps == kAdjWarps, "one launch helper");
+    const int T = 2 * a.K + 1, Ns = a.M - L + 1;
+    const long long units = ((long long)a.Nx * a.Ny + kRowWarps - 1) / kRowWarps;
+    auto cost = [&](int sb) { return (T * ((Ns + sb - 1) / sb) + 31) / 32 * (sb + 2); };
+    auto go = [&](auto kern, int sb) {
+        return launch_adjoint_with(kern, a, units, AdjRowSmem(a.M, L, T, sb).total, num_sms, s);
+    };
+    int best = 2;
+    for (int sb : {4, 6, 8})
+        if (cost(sb) < cost(best)) best = sb;
+    return best == 2   ? go(adjoint_row_kernel<L, 2>, 2)
+           : best == 4 ? go(adjoint_row_kernel<L, 4>, 4)
+           : best == 6 ? go(adjoint_row_kernel<L, 6>, 6)
+                       : go(adjoint_row_kernel<L, 8>, 8);
 }
 
 int launch_adjoint(const AdjDev &a, int num_sms, cudaStream_t s)
@@ -283,16 +371,19 @@ int launch_adjoint(const AdjDev &a, int num_sms, cudaStream_t s)
     const size_t smem = (size_t)2 * rows * a.M * sizeof(float2) + (size_t)((a.M + 1) & ~1) * sizeof(float) +
                         (size_t)kAdjWarps * (a.L + T * Ns) * sizeof(float2);
     if (smem > 227 * 1024 || a.L > 64) return cudaErrorNotSupported;
-    const size_t smem_b = smem + (size_t)2 * rows * kAdjPad * sizeof(float2);  // padded rows
-    if (smem_b <= 227 * 1024) {
+    // rows where they leave two CTAs an SM; the tiles serve the other lengths,
+    // very long windows and very wide apertures
+    if (T <= 32 && AdjRowSmem(a.M, a.L, T, 8).total <= 112 * 1024) {
         switch (a.L) {
-        case 8: return launch_adjoint_with(adjoint_blocked_kernel<8>, a, smem_b, num_sms, s);
-        case 16: return launch_adjoint_with(adjoint_blocked_kernel<16>, a, smem_b, num_sms, s);
-        case 32: return launch_adjoint_with(adjoint_blocked_kernel<32>, a, smem_b, num_sms, s);
+        case 8: return launch_rows<8>(a, num_sms, s);
+        case 16: return launch_rows<16>(a, num_sms, s);
+        case 24: return launch_rows<24>(a, num_sms, s);
+        case 32: return launch_rows<32>(a, num_sms, s);
         default: break;
         }
     }
-    return launch_adjoint_with(adjoint_kernel, a, smem, num_sms, s);
+    const long long units = (long long)a.Nx * ((a.Npy + kAdjTile - 1) / kAdjTile);
+    return launch_adjoint_with(adjoint_kernel, a, units, smem, num_sms, s);
 }
 
 }  // namespace cgb
