@@ -68,9 +68,10 @@ static __device__ __noinline__ void stall_test_exit(unsigned *status, uint64_t *
 // code into an immediate); SYNC: barrier points that keep the CTA's warps in
 // step, so that the long unrolled instruction stream is fetched once for all
 // of them.
-template <int L_, int G_, int WARPS_, int NITER_, int T_, int M_, bool SYNC_, bool WIDE_ = (L_ > 32)>
+// BLOCKS: CTAs an SM the registers are held to.
+template <int L_, int G_, int WARPS_, int NITER_, int T_, int M_, bool SYNC_, bool WIDE_ = (L_ > 32), int BLOCKS_ = 1>
 struct Cfg {
-    static constexpr int L = L_, G = G_, WARPS = WARPS_, NITER = NITER_, M = M_;
+    static constexpr int L = L_, G = G_, WARPS = WARPS_, NITER = NITER_, M = M_, BLOCKS = BLOCKS_;
     // RT_T: T from the frame; T then sizes only the unused L <= 32 code
     static constexpr bool RT_T = T_ == 0;
     static constexpr int T = RT_T ? 1 : T_;
@@ -124,7 +125,7 @@ COS_DEV int unit_frame(const FramesParam &fp, long long u)
 // MODE (FusedMode): z/P, z/P and w, or R alone; each mode carries only its
 // own output code, so its unrolled instruction stream stays small.
 template <class C, int MODE>
-__global__ void __launch_bounds__(C::WARPS * 32, 1)
+__global__ void __launch_bounds__(C::WARPS * 32, C::BLOCKS)
 fused_kernel(const __grid_constant__ FramesParam fp, long long total_units, unsigned *status)
 {
     constexpr int L = C::L, G = C::G, NM = C::NM, PPW = C::PPW, TILE = C::TILE, T = C::T;
