@@ -138,6 +138,9 @@ COS_DEV void wide_pixel(const FrameDev &f, const float4 *xw, const int XS, const
     // the w and the refinement modes carry the right-hand side a only and keep
     // the factor for the back substitution
     constexpr bool WMODE = MODE == FUSED_W || MODE == FUSED_REFINE;
+    // the lock-step barriers are CTA-wide, and the refinement pass of the adaptive
+    // mode (OWN_R0) is taken by some of a CTA's warps only: it has none
+    constexpr bool SYNC = C::SYNC && !OWN_R0;
     using WA = WideArea<L, G>;
     using WS = WideStash<L, G>;
     static_assert(WA::Q <= C::RBQ && (G * (G + 1) + 1) / 2 <= C::RBQ && (L + 1) / 2 + 8 * G <= C::RBQ,
@@ -339,7 +342,7 @@ COS_DEV void wide_pixel(const FrameDev &f, const float4 *xw, const int XS, const
 
         // SYNC: barriers at fixed points of the unrolled code keep the CTA's
         // warps in step, so that each stretch of it is fetched once for all
-        if (C::SYNC) __syncthreads();
+        if (SYNC) __syncthreads();
         // ---- 2. loading on the block's diagonal (row b*G + r, slot b)
 #pragma unroll
         for (int q = 0; q < G; ++q)
@@ -397,7 +400,7 @@ COS_DEV void wide_pixel(const FrameDev &f, const float4 *xw, const int XS, const
                         A[b * G + q][m] = ffma2(vii[m], make_float2(u4.z, u4.w),
                                                 ffma2(vrr[m], make_float2(u4.x, u4.y), A[b * G + q][m]));
                 }
-                if (C::SYNC && p % 8 == 7) __syncthreads();
+                if (SYNC && p % 8 == 7) __syncthreads();
             });
 
             // ---- 4. the block's factorisation steps
@@ -454,7 +457,7 @@ COS_DEV void wide_pixel(const FrameDev &f, const float4 *xw, const int XS, const
                     for (int m = b; m < NM; ++m)
                         A[k][m] = ffma2(vii[m], make_float2(u4.z, u4.w), ffma2(vrr[m], make_float2(u4.x, u4.y), A[k][m]));
                 }
-                if (C::SYNC && i % 8 == 7) __syncthreads();
+                if (SYNC && i % 8 == 7) __syncthreads();
             });
         }
     });
