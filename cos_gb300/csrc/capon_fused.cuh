@@ -68,10 +68,14 @@ static __device__ __noinline__ void stall_test_exit(unsigned *status, uint64_t *
 // code into an immediate); SYNC: barrier points that keep the CTA's warps in
 // step, so that the long unrolled instruction stream is fetched once for all
 // of them.
-// BLOCKS: CTAs an SM the registers are held to.
-template <int L_, int G_, int WARPS_, int NITER_, int T_, int M_, bool SYNC_, bool WIDE_ = (L_ > 32), int BLOCKS_ = 1>
+// BLOCKS: CTAs an SM the registers are held to.  XS: with M taken at run time, a
+// compile-time row stride for every M <= XS - 2 (0: M + 2), which turns the
+// window's row offsets back into immediates; only the offset of the last
+// subarray, Ns, stays in a register.
+template <int L_, int G_, int WARPS_, int NITER_, int T_, int M_, bool SYNC_, bool WIDE_ = (L_ > 32), int BLOCKS_ = 1,
+          int XS_ = 0>
 struct Cfg {
-    static constexpr int L = L_, G = G_, WARPS = WARPS_, NITER = NITER_, M = M_, BLOCKS = BLOCKS_;
+    static constexpr int L = L_, G = G_, WARPS = WARPS_, NITER = NITER_, M = M_, BLOCKS = BLOCKS_, XS = XS_;
     // RT_T: T from the frame; T then sizes only the unused L <= 32 code
     static constexpr bool RT_T = T_ == 0;
     static constexpr int T = RT_T ? 1 : T_;
@@ -98,10 +102,10 @@ struct Cfg {
 struct Smem {
     int rows, XS;  // tile rows (TILE+2K), expanded row stride (quads)
     size_t off_raw0, off_raw1, off_xe, off_c, off_g, off_rb, off_bar, total;
-    __host__ __device__ Smem(int TILE, int K, int M, int L, int WARPS, int PPW, int RBQ)
+    __host__ __device__ Smem(int TILE, int K, int M, int L, int WARPS, int PPW, int RBQ, int XS_)
     {
         rows = TILE + 2 * K;
-        XS = M + 2;
+        XS = XS_ ? XS_ : M + 2;
         const size_t raw = ((size_t)rows * M * sizeof(float2) + 127) & ~(size_t)127;
         off_raw0 = 0;
         off_raw1 = off_raw0 + raw;
@@ -138,7 +142,7 @@ fused_kernel(const __grid_constant__ FramesParam fp, long long total_units, unsi
     // carve-up; the host groups frames so that K and M are equal within a launch
     const FrameDev &f0 = fp.f[0];
     const int K = C::RT_T ? f0.K : (C::T - 1) / 2;
-    const Smem S(TILE, K, C::M ? C::M : f0.M, L, C::WARPS, PPW, C::RBQ);
+    const Smem S(TILE, K, C::M ? C::M : f0.M, L, C::WARPS, PPW, C::RBQ, C::XS);
     float2 *raw[2] = {(float2 *)(smem + S.off_raw0), (float2 *)(smem + S.off_raw1)};
     float4 *xe = (float4 *)(smem + S.off_xe);
     float2 *cs = (float2 *)(smem + S.off_c);
@@ -194,7 +198,7 @@ fused_kernel(const __grid_constant__ FramesParam fp, long long total_units, unsi
         const int bx = (int)(lu / f.tiles_per_beam);
         const int p0 = (int)(lu % f.tiles_per_beam) * TILE;
         const int rows = min(TILE + 2 * K, f.Ny - p0);
-        const int XS = M + 2;
+        const int XS = C::XS ? C::XS : M + 2;
 
         const bool ok = mbar_wait_bounded(&bar[b], b ? ph1 : ph0);
         if (b) ph1 ^= 1u; else ph0 ^= 1u;
@@ -206,9 +210,11 @@ fused_kernel(const __grid_constant__ FramesParam fp, long long total_units, unsi
         const bool direct = ((((size_t)rows * M * sizeof(float2)) & 15u) != 0) || ((((uintptr_t)src) & 15u) != 0);
 
         // ---- expand rows to quads; per-row first covariance row c and subarray sums g
+        const float invM = 1.0f / (float)M;
         for (int i = tid; i < rows * M; i += nthreads) {
             const float2 v = direct ? src[i] : raw[b][i];
-            const int rr = i / M, cc = i % M;
+            // i / M: by the reciprocal (exact below 2^21) where M is not a constant
+            const int rr = C::M ? i / M : (int)(((float)i + 0.5f) * invM), cc = C::M ? i % M : i - rr * M;
             xe[rr * XS + cc] = make_float4(v.x, v.y, v.y, -v.x);
         }
         __syncthreads();
@@ -250,7 +256,7 @@ fused_kernel(const __grid_constant__ FramesParam fp, long long total_units, unsi
                     w1 = w2;
                     w2 = w3;
                 }
-            } else {
+            } else if constexpr (C::M != 0) {
                 // three chunks per iteration: enough independent work to cover the
                 // load and TwoSum latencies, without the code growth of a full
                 // unroll (which slows the unrolled per-pixel phases that follow
@@ -280,6 +286,39 @@ fused_kernel(const __grid_constant__ FramesParam fp, long long total_units, unsi
 #pragma unroll
                     for (int q = 0; q < 4; ++q) two_sum_acc(hi[q], lo[q], make_float2(P[q].x + P[q].y, Q[q].x + Q[q].y));
                 }
+            } else {
+                // the same sums with Ns at run time: whole chunks without a test for
+                // every term, then the last one (2.31 -> 2.17 ms at M=60, L=32, K=2;
+                // the constant Ns keeps the loop above, 0.6 % faster there)
+                // chunk s0 .. s0+3; FULL: all four terms exist
+                auto chunk = [&](const int s0, auto full) __attribute__((always_inline)) {
+                    float2 P[4], Q[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) P[q] = Q[q] = make_float2(0.f, 0.f);
+#pragma unroll
+                    for (int ss = 0; ss < 4; ++ss) {
+                        const int s = s0 + ss;
+                        if (decltype(full)::value || s < Ns) {
+                            const float4 a = xr[s], w3 = xr[s + j0 + 3];
+                            const float4 c[4] = {w0, w1, w2, w3};
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) {
+                                P[q] = ffma2(make_float2(a.x, a.y), make_float2(c[q].x, c[q].y), P[q]);
+                                Q[q] = ffma2(make_float2(a.z, a.w), make_float2(c[q].x, c[q].y), Q[q]);
+                            }
+                            w0 = w1;
+                            w1 = w2;
+                            w2 = w3;
+                        }
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        two_sum_acc(hi[q], lo[q], make_float2(P[q].x + P[q].y, Q[q].x + Q[q].y));
+                };
+                const int whole = Ns & ~3;
+#pragma unroll 3
+                for (int s0 = 0; s0 < whole; s0 += 4) chunk(s0, std::true_type{});
+                if (whole < Ns) chunk(whole, std::false_type{});
             }
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -735,7 +774,8 @@ fused_kernel(const __grid_constant__ FramesParam fp, long long total_units, unsi
 template <class C>
 size_t smem_bytes(int K, int M)
 {
-    return Smem(C::TILE, K, C::M ? C::M : M, C::L, C::WARPS, C::PPW, C::RBQ).total;
+    if (C::XS && M + 2 > C::XS) return SIZE_MAX;  // the row does not fit the stride: not for this M
+    return Smem(C::TILE, K, C::M ? C::M : M, C::L, C::WARPS, C::PPW, C::RBQ, C::XS).total;
 }
 
 // bytes of FramesParam::stash the refinement mode needs on num_sms SMs
@@ -763,7 +803,7 @@ int launch_cfg(FramesParam fp, unsigned *status, int num_sms, cudaStream_t s)
     const FrameDev &f0 = fp.f[0];
     if (!C::RT_T && 2 * f0.K + 1 != C::T) return cudaErrorNotSupported;
     for (int i = 0; i < fp.n; ++i)
-        if (C::M && fp.f[i].M != C::M) return cudaErrorNotSupported;
+        if ((C::M && fp.f[i].M != C::M) || (C::XS && fp.f[i].M + 2 > C::XS)) return cudaErrorNotSupported;
     long long begin = 0;
     for (int i = 0; i < fp.n; ++i) {
         FrameDev &g = fp.f[i];
@@ -772,7 +812,7 @@ int launch_cfg(FramesParam fp, unsigned *status, int num_sms, cudaStream_t s)
         g.tile_begin = begin;
         begin += (long long)g.Nx * g.tiles_per_beam;
     }
-    Smem S(C::TILE, f0.K, C::M ? C::M : f0.M, C::L, C::WARPS, C::PPW, C::RBQ);
+    Smem S(C::TILE, f0.K, C::M ? C::M : f0.M, C::L, C::WARPS, C::PPW, C::RBQ, C::XS);
     if (S.total > kFusedSmemMax) return cudaErrorNotSupported;
     cudaError_t e = cudaFuncSetAttribute(fused_kernel<C, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)S.total);
