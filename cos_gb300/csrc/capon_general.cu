@@ -59,22 +59,32 @@ constexpr int kCovMaxM = 1020;       // i / 4 fits a byte of the block table
 struct CovShape {
     int tile;        // pixels per unit
     int seg, nseg;   // pixels per product item, items along the tile
-    int XS, LS, M4;  // sample row stride, row stride of q and of R, rows of q
+    int XS, LS;      // sample row stride; row stride of q up to row Ns - 1
+    int QS;          // entries of q a pixel holds
     int blocks;      // (i, d) blocks that hold an entry
-    size_t off_q, off_tab, total;
+    size_t off_q, off_tab, off_row, total;
     __host__ __device__ CovShape(int tile_, int K, int M, int L)
     {
         tile = tile_;
         seg = tile;
         nseg = 1;
-        M4 = (M + 3) & ~3;
         LS = (L + 1) & ~1;
+        QS = row(M, M, L);
         XS = (M + 6 + 1) & ~1;  // a block reads up to 5 samples past its last valid column
         blocks = 0;
-        for (int i = 0; i < M4; i += 4) blocks += cols(i, M);
+        for (int i = 0; i < M; i += 4) blocks += cols(i, M);
         off_q = (size_t)(tile + 2 * K) * XS * sizeof(float2);
-        off_tab = off_q + (size_t)tile * M4 * LS * sizeof(float2);
-        total = off_tab + (((size_t)blocks * sizeof(unsigned short) + 15) & ~(size_t)15);
+        // LS entries past the last pixel's: lanes past a diagonal's end read on
+        off_tab = off_q + ((size_t)tile * QS + LS) * sizeof(float2);
+        off_row = off_tab + (((size_t)blocks * sizeof(unsigned short) + 15) & ~(size_t)15);
+        total = off_row + (((size_t)(M + 4) * sizeof(int) + 15) & ~(size_t)15);
+    }
+    // offset of row i of q: LS entries up to row Ns - 1, then as many as the row
+    // holds (i + d < M), rounded up to pairs
+    __host__ __device__ int row(int i, int M, int L) const
+    {
+        const int Ns = M - L + 1;
+        return i <= Ns ? i * LS : Ns * LS + Record::row(i - Ns, L - 1);
     }
     // 2-column blocks of the rows i .. i+3 that hold an entry i + d < M
     __host__ __device__ int cols(int i, int M) const { return LS / 2 < (M - i + 1) / 2 ? LS / 2 : (M - i + 1) / 2; }
@@ -114,12 +124,14 @@ cov_kernel(FrameDev f, CovShape S, float2 *__restrict__ work, int units)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     const int M = f.M, L = f.L, K = T_ ? (T_ - 1) / 2 : f.K, T = 2 * K + 1, Ns = M - L + 1;
-    const int XS = S.XS, LS = S.LS, M4 = S.M4, tid = threadIdx.x, rec = Record::size(L);
+    const int XS = S.XS, LS = S.LS, QS = S.QS, tid = threadIdx.x, rec = Record::size(L);
     float2 *xs = (float2 *)smraw;
     float2 *qs = (float2 *)(smraw + S.off_q);
     unsigned short *tab = (unsigned short *)(smraw + S.off_tab);
+    int *rowq = (int *)(smraw + S.off_row);   // offsets of the rows of q
+    for (int i = tid; i < M; i += kCovThreads) rowq[i] = S.row(i, M, L);
     // the (i, d) blocks, dense: (i/4) << 8 | d/2
-    for (int t = tid; t < (M4 / 4) * (LS / 2); t += kCovThreads) {
+    for (int t = tid; t < (M + 3) / 4 * (LS / 2); t += kCovThreads) {
         const int a = t / (LS / 2), b = t % (LS / 2);
         if (b >= S.cols(4 * a, M)) continue;
         int off = b;
@@ -151,12 +163,16 @@ cov_kernel(FrameDev f, CovShape S, float2 *__restrict__ work, int units)
             const int sg = small_div(it, inv_blocks), e = tab[it - sg * S.blocks];
             const int i0 = (e >> 8) * 4, d0 = (e & 255) * 2, s0 = sg * S.seg, sp = min(S.seg, np - s0);
             const float2 *xi = xs + s0 * XS + i0, *xj = xi + d0;
-            float2 *qd = qs + ((size_t)s0 * M4 + i0) * LS + d0;
+            float2 *qd = qs + (size_t)s0 * QS + d0;
+            int ro[4];   // -1: the row has no entry in these columns
+#pragma unroll
+            for (int a = 0; a < 4; ++a) ro[a] = i0 + a + d0 < M ? rowq[i0 + a] : -1;
             auto put = [&](const float2(&v)[8]) __attribute__((always_inline)) {
 #pragma unroll
                 for (int a = 0; a < 4; ++a)
-                    *(float4 *)(qd + a * LS) = make_float4(v[2 * a].x, v[2 * a].y, v[2 * a + 1].x, v[2 * a + 1].y);
-                qd += M4 * LS;
+                    if (ro[a] >= 0)
+                        *(float4 *)(qd + ro[a]) = make_float4(v[2 * a].x, v[2 * a].y, v[2 * a + 1].x, v[2 * a + 1].y);
+                qd += QS;
             };
             if constexpr (T_ != 0) {
                 float2 ring[T_][8];
@@ -218,7 +234,7 @@ cov_kernel(FrameDev f, CovShape S, float2 *__restrict__ work, int units)
         for (int p = tid >> 5; p < np; p += kCovThreads / 32) {
             float h = 0.f, l = 0.f;
             for (int i = tid & 31; i < M; i += 32) {
-                const float c = (float)min(min(i + 1, M - i), min(L, Ns)), v = qs[((size_t)p * M4 + i) * LS].x;
+                const float c = (float)min(min(i + 1, M - i), min(L, Ns)), v = qs[(size_t)p * QS + rowq[i]].x;
                 const float pr = c * v, s = h + pr, bb = s - h;
                 l += (h - (s - bb)) + (pr - bb) + fmaf(c, v, -pr);
                 h = s;
@@ -240,11 +256,12 @@ cov_kernel(FrameDev f, CovShape S, float2 *__restrict__ work, int units)
 #pragma unroll 1
         for (int it = tid; it < np * L; it += kCovThreads) {
             const int p = small_div(it, inv_L), d = it - p * L, n = L - d;
-            const float2 *q = qs + (size_t)p * M4 * LS + d;
+            const float2 *q = qs + (size_t)p * QS + d;
             float2 *out = work + (pix0 + p) * rec + d;
-            // forward-backward: q_d[i] + q_d[M-1-d-i] takes q's place, halved at the store
-            auto term = [&](int i) __attribute__((always_inline)) {
-                return FB ? fadd2(q[i * LS], q[max(M - 1 - d - i, 0) * LS]) : q[i * LS];
+            // entry i of the diagonal, at offset o; forward-backward: q_d[i] + q_d[M-1-d-i]
+            // takes its place, halved at the store
+            auto term = [&](int i, int o) __attribute__((always_inline)) {
+                return FB ? fadd2(q[o], q[rowq[max(M - 1 - d - i, 0)]]) : q[o];
             };
             float2 h = make_float2(0.f, 0.f), l = h;
             {
@@ -253,10 +270,10 @@ cov_kernel(FrameDev f, CovShape S, float2 *__restrict__ work, int units)
                 int i = 0;
 #pragma unroll 4
                 for (; i + 1 < Ns; i += 2) {
-                    two_sum_acc(h, l, term(i));
-                    two_sum_acc(h1, l1, term(i + 1));
+                    two_sum_acc(h, l, term(i, i * LS));
+                    two_sum_acc(h1, l1, term(i + 1, (i + 1) * LS));
                 }
-                if (i < Ns) two_sum_acc(h, l, term(i));
+                if (i < Ns) two_sum_acc(h, l, term(i, i * LS));
                 two_sum_acc(h, l, h1);
                 l = fadd2(l, l1);
             }
@@ -265,9 +282,10 @@ cov_kernel(FrameDev f, CovShape S, float2 *__restrict__ work, int units)
                 float2 add[4], sub[4];
 #pragma unroll
                 for (int v = 0; v < 4; ++v) {
-                    const int i = min(k0 + v, max(L - 2, 0));  // the last row's step is not used
-                    add[v] = term(i + (L > 1 ? Ns : 0));
-                    sub[v] = term(i);
+                    // the last row's step is not used
+                    const int i = min(k0 + v, max(L - 2, 0)), j = L > 1 ? i + Ns : 0;
+                    add[v] = term(j, rowq[j]);
+                    sub[v] = term(i, rowq[i]);
                 }
 #pragma unroll
                 for (int v = 0; v < 4; ++v) {
@@ -308,8 +326,10 @@ CovShape cov_shape(const FrameDev &f, int num_sms)
     const int T = 2 * f.K + 1;
     const CovShape one(1, f.K, f.M, f.L);
     if (one.total > 226 * 1024) return CovShape(0, f.K, f.M, f.L);
-    const size_t per = ((size_t)one.XS + (size_t)one.M4 * one.LS) * sizeof(float2);
-    auto room = [&](size_t most) { return one.total > most ? 0 : 1 + (int)std::min<size_t>(63, (most - one.total) / per); };
+    const size_t per = ((size_t)one.XS + (size_t)one.QS) * sizeof(float2);
+    auto room = [&](size_t most) {
+        return one.total > most ? 0 : 1 + (int)std::min<size_t>(63, (most - one.total) / per);
+    };
     int tile = room(112 * 1024);
     if (tile < 4) tile = room(226 * 1024);
     const long long npix = (long long)f.Nx * f.Npy;
@@ -369,7 +389,8 @@ int launch_general(const FrameDev &f, float2 *work, unsigned *status, int num_sm
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S.total);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kCovThreads, S.total)) != cudaSuccess) return e;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kCovThreads, S.total);
+    if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorNotSupported;
     const long long grid = std::min<long long>(units, (long long)num_sms * per_sm);
     kern<<<(unsigned)grid, kCovThreads, S.total, s>>>(f, S, work, (int)units);
