@@ -726,6 +726,7 @@ int cos_capon_tdib(cos_capon_ctx *c, const void *mfdata, int n_hydros, int n_sam
     memset(&t, 0, sizeof(t));
     t.t0 = t0;
     t.dt = dt;
+    t.inv_dt = 1.0 / dt;
     t.inv_c = 1.0 / cs;
     t.fc = fc;
     t.n_hydros = n_hydros;
