@@ -10,6 +10,8 @@ int fused_l48a_launch(const FramesParam &fp, int mode, unsigned *st, int n, cuda
 int fused_l48a_launch_refine(const FramesParam &fp, int mode, unsigned *st, int n, cudaStream_t s);
 size_t fused_l48a_smem(int K, int M);
 size_t fused_l48a_stash(int num_sms);
+int fused_l48b_launch(const FramesParam &fp, int mode, unsigned *st, int n, cudaStream_t s);
+size_t fused_l48b_smem(int K, int M);
 
 namespace {
 int launch_l48a(const FramesParam &fp, int mode, unsigned *st, int n, cudaStream_t s)
@@ -18,6 +20,9 @@ int launch_l48a(const FramesParam &fp, int mode, unsigned *st, int n, cudaStream
 }
 
 const FusedCandidate kCand[] = {
+    // z/P, w and R: 12 warps at 168 registers (K=1, M=96, 262 k pixels: z and P 4.89 ->
+    // 3.69 ms, w 5.30 -> 4.33); refinement keeps 8 warps (11.8 ms against 14.8)
+    {"L48.G16.W12.N1", 48, 0, 0, fused_l48b_launch, fused_l48b_smem},
     {"L48.G16.W8.N1.sync", 48, 0, 0, launch_l48a, fused_l48a_smem, fused_l48a_stash},
 };
 }  // namespace

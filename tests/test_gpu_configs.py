@@ -49,3 +49,10 @@ def test_four_warp_candidates(rows, K, M, monkeypatch):
 def test_stride_66_candidates(rows, K, M, monkeypatch):
     T = 2 * K + 1
     check(32, K, M, rows, [f"L32.G8.W8.N2.X66.T{T}"], f"L32.G8.W8.N2.sync.T{T}", monkeypatch)
+
+
+@pytest.mark.parametrize("M", [48, 61, 97])
+@pytest.mark.parametrize("K", [0, 1, 4])
+@pytest.mark.parametrize("rows", [1, 23, 25])
+def test_twelve_warp_l48(rows, K, M, monkeypatch):
+    check(48, K, M, rows, ["L48.G16.W12.N1"], "L48.G16.W8.N1.sync", monkeypatch)
