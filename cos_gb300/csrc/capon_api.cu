@@ -417,7 +417,7 @@ static int run_frames(cos_capon_ctx *c, const FrameDev *fs, int n, const cos_cap
             return e;
         }
         // element space without a fused instantiation: the general path where it
-        // serves the frame, else (refinement, few subarrays) the precise
+        // serves the frame, else (refinement) the precise
         // pipeline; the plain form when asked for
         return is_tc_form(o.form)                              ? run_tc(c, f, o.form, o.refine != 0, st)
                : (o.form == COS_CAPON_FORM_PLAIN && !o.refine) ? run_plain(c, f, st)

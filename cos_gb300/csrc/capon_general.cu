@@ -36,6 +36,7 @@
 // precise pipeline, 0.17 ms here + 0.12 ms in the solve stage; 65 k pixels at
 // M=64, L=32, K=2 with forward-backward averaging: 2.56 ms, 0.38 + 0.17 ms.
 #include <algorithm>
+#include <type_traits>
 
 #include "capon_common.cuh"
 #include "capon_general.cuh"
@@ -61,11 +62,13 @@ struct CovShape {
     int seg, nseg;   // pixels per product item, items along the tile
     int XS, LS;      // sample row stride; row stride of q up to row Ns - 1
     int QS;          // entries of q a pixel holds
+    int EB;          // bytes of an entry: 8, or 16 for the exact form (value and remainder)
     int blocks;      // (i, d) blocks that hold an entry
     size_t off_q, off_tab, off_row, total;
-    __host__ __device__ CovShape(int tile_, int K, int M, int L)
+    __host__ __device__ CovShape(int tile_, int K, int M, int L, bool exact)
     {
         tile = tile_;
+        EB = exact ? 16 : 8;
         seg = tile;
         nseg = 1;
         LS = (L + 1) & ~1;
@@ -75,7 +78,7 @@ struct CovShape {
         for (int i = 0; i < M; i += 4) blocks += cols(i, M);
         off_q = (size_t)(tile + 2 * K) * XS * sizeof(float2);
         // LS entries past the last pixel's: lanes past a diagonal's end read on
-        off_tab = off_q + ((size_t)tile * QS + LS) * sizeof(float2);
+        off_tab = off_q + ((size_t)tile * QS + LS) * EB;
         off_row = off_tab + (((size_t)blocks * sizeof(unsigned short) + 15) & ~(size_t)15);
         total = off_row + (((size_t)(M + 4) * sizeof(int) + 15) & ~(size_t)15);
     }
@@ -116,9 +119,29 @@ COS_DEV void block_products(float2 (&out)[8], const float2 *xi, const float2 *xj
     }
 }
 
+// the same added to the float-float (h, l), every product exact (TwoProd by fma)
+COS_DEV void block_products_exact(float2 (&h)[8], float2 (&l)[8], const float2 *xi, const float2 *xj)
+{
+    const float2 z = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const float2 a = xi[q], as = make_float2(a.y, -a.x);
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            const float2 v = xj[q + b], vr = make_float2(v.x, v.x), vi = make_float2(v.y, v.y);
+            const float2 p1 = ffma2(vr, a, z), p2 = ffma2(vi, as, z);
+            const float2 e1 = ffma2(vr, a, make_float2(-p1.x, -p1.y)), e2 = ffma2(vi, as, make_float2(-p2.x, -p2.y));
+            two_sum_acc(h[2 * q + b], l[2 * q + b], p1);
+            two_sum_acc(h[2 * q + b], l[2 * q + b], p2);
+            l[2 * q + b] = fadd2(l[2 * q + b], fadd2(e1, e2));
+        }
+    }
+}
+
 // T: the temporal window 2K+1, 0 = taken from the frame (products formed anew
-// for every pixel of the window: the row ring needs a compile-time length)
-template <int T_, bool FB>
+// for every pixel of the window: the row ring needs a compile-time length).
+// EXACT (T = 0): q and everything after it in float-float, the products exact.
+template <int T_, bool FB, bool EXACT = false>
 __global__ void __launch_bounds__(kCovThreads, 2)
 cov_kernel(FrameDev f, CovShape S, float2 *__restrict__ work, int units)
 {
@@ -126,7 +149,9 @@ cov_kernel(FrameDev f, CovShape S, float2 *__restrict__ work, int units)
     const int M = f.M, L = f.L, K = T_ ? (T_ - 1) / 2 : f.K, T = 2 * K + 1, Ns = M - L + 1;
     const int XS = S.XS, LS = S.LS, QS = S.QS, tid = threadIdx.x, rec = Record::size(L);
     float2 *xs = (float2 *)smraw;
-    float2 *qs = (float2 *)(smraw + S.off_q);
+    static_assert(!EXACT || T_ == 0, "the exact form takes any window");
+    using Entry = typename std::conditional<EXACT, float4, float2>::type;   // (value, remainder) or the value
+    Entry *qs = (Entry *)(smraw + S.off_q);
     unsigned short *tab = (unsigned short *)(smraw + S.off_tab);
     int *rowq = (int *)(smraw + S.off_row);   // offsets of the rows of q
     for (int i = tid; i < M; i += kCovThreads) rowq[i] = S.row(i, M, L);
@@ -163,7 +188,7 @@ cov_kernel(FrameDev f, CovShape S, float2 *__restrict__ work, int units)
             const int sg = small_div(it, inv_blocks), e = tab[it - sg * S.blocks];
             const int i0 = (e >> 8) * 4, d0 = (e & 255) * 2, s0 = sg * S.seg, sp = min(S.seg, np - s0);
             const float2 *xi = xs + s0 * XS + i0, *xj = xi + d0;
-            float2 *qd = qs + (size_t)s0 * QS + d0;
+            Entry *qd = qs + (size_t)s0 * QS + d0;
             int ro[4];   // -1: the row has no entry in these columns
 #pragma unroll
             for (int a = 0; a < 4; ++a) ro[a] = i0 + a + d0 < M ? rowq[i0 + a] : -1;
@@ -174,7 +199,22 @@ cov_kernel(FrameDev f, CovShape S, float2 *__restrict__ work, int units)
                         *(float4 *)(qd + ro[a]) = make_float4(v[2 * a].x, v[2 * a].y, v[2 * a + 1].x, v[2 * a + 1].y);
                 qd += QS;
             };
-            if constexpr (T_ != 0) {
+            if constexpr (EXACT) {
+#pragma unroll 1
+                for (int p = 0; p < sp; ++p) {
+                    float2 h[8], l[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) h[q] = l[q] = make_float2(0.f, 0.f);
+#pragma unroll 1
+                    for (int t = 0; t < T; ++t) block_products_exact(h, l, xi + (p + t) * XS, xj + (p + t) * XS);
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const float2 v = fadd2(h[q], l[q]), e = fsub2(l[q], fsub2(v, h[q]));
+                        if (ro[q / 2] >= 0) qd[ro[q / 2] + q % 2] = make_float4(v.x, v.y, e.x, e.y);
+                    }
+                    qd += QS;
+                }
+            } else if constexpr (T_ != 0) {
                 float2 ring[T_][8];
                 const int nr = sp + T_ - 1;
 #pragma unroll 1
@@ -234,9 +274,11 @@ cov_kernel(FrameDev f, CovShape S, float2 *__restrict__ work, int units)
         for (int p = tid >> 5; p < np; p += kCovThreads / 32) {
             float h = 0.f, l = 0.f;
             for (int i = tid & 31; i < M; i += 32) {
-                const float c = (float)min(min(i + 1, M - i), min(L, Ns)), v = qs[(size_t)p * QS + rowq[i]].x;
+                const Entry e = qs[(size_t)p * QS + rowq[i]];
+                const float c = (float)min(min(i + 1, M - i), min(L, Ns)), v = e.x;
                 const float pr = c * v, s = h + pr, bb = s - h;
                 l += (h - (s - bb)) + (pr - bb) + fmaf(c, v, -pr);
+                if constexpr (EXACT) l = fmaf(c, e.z, l);
                 h = s;
             }
             for (int o = 16; o; o >>= 1) {
@@ -256,45 +298,73 @@ cov_kernel(FrameDev f, CovShape S, float2 *__restrict__ work, int units)
 #pragma unroll 1
         for (int it = tid; it < np * L; it += kCovThreads) {
             const int p = small_div(it, inv_L), d = it - p * L, n = L - d;
-            const float2 *q = qs + (size_t)p * QS + d;
+            const Entry *q = qs + (size_t)p * QS + d;
             float2 *out = work + (pix0 + p) * rec + d;
-            // entry i of the diagonal, at offset o; forward-backward: q_d[i] + q_d[M-1-d-i]
-            // takes its place, halved at the store
-            auto term = [&](int i, int o) __attribute__((always_inline)) {
-                return FB ? fadd2(q[o], q[rowq[max(M - 1 - d - i, 0)]]) : q[o];
-            };
-            float2 h = make_float2(0.f, 0.f), l = h;
-            {
-                // q[0] + .. + q[Ns-1] on two chains
-                float2 h1 = h, l1 = h;
-                int i = 0;
-#pragma unroll 4
-                for (; i + 1 < Ns; i += 2) {
-                    two_sum_acc(h, l, term(i, i * LS));
-                    two_sum_acc(h1, l1, term(i + 1, (i + 1) * LS));
-                }
-                if (i < Ns) two_sum_acc(h, l, term(i, i * LS));
-                two_sum_acc(h, l, h1);
-                l = fadd2(l, l1);
-            }
-#pragma unroll 1
-            for (int k0 = 0; k0 < L; k0 += 4) {
-                float2 add[4], sub[4];
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    // the last row's step is not used
-                    const int i = min(k0 + v, max(L - 2, 0)), j = L > 1 ? i + Ns : 0;
-                    add[v] = term(j, rowq[j]);
-                    sub[v] = term(i, rowq[i]);
-                }
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
+            if constexpr (EXACT) {
+                float2 h = make_float2(0.f, 0.f), l = h;
+                // (h, l) += sign times entry i (and its mirror: halved at the store)
+                auto add = [&](int i, float sign) __attribute__((always_inline)) {
+                    float4 e = q[rowq[i]];
+                    two_sum_acc(h, l, make_float2(sign * e.x, sign * e.y));
+                    l = fadd2(l, make_float2(sign * e.z, sign * e.w));
+                    if (FB) {
+                        e = q[rowq[max(M - 1 - d - i, 0)]];
+                        two_sum_acc(h, l, make_float2(sign * e.x, sign * e.y));
+                        l = fadd2(l, make_float2(sign * e.z, sign * e.w));
+                    }
+                };
+#pragma unroll 2
+                for (int i = 0; i < Ns; ++i) add(i, 1.f);
+#pragma unroll 2
+                for (int k = 0; k < L; ++k) {
                     float2 r = fadd2(h, l);
                     if (FB) r = cscale(r, 0.5f);
-                    if (k0 + v < n) *out = r;
-                    out += (L - k0 - v + 1) & ~1;
-                    two_sum_acc(h, l, add[v]);
-                    two_sum_acc(h, l, make_float2(-sub[v].x, -sub[v].y));
+                    if (k < n) *out = r;
+                    out += (L - k + 1) & ~1;
+                    if (k + 1 < L) {
+                        add(k + Ns, 1.f);
+                        add(k, -1.f);
+                    }
+                }
+            } else {
+                // entry i of the diagonal, at offset o; forward-backward: q_d[i] + q_d[M-1-d-i]
+                // takes its place, halved at the store
+                auto term = [&](int i, int o) __attribute__((always_inline)) {
+                    return FB ? fadd2(q[o], q[rowq[max(M - 1 - d - i, 0)]]) : q[o];
+                };
+                float2 h = make_float2(0.f, 0.f), l = h;
+                {
+                    // q[0] + .. + q[Ns-1] on two chains
+                    float2 h1 = h, l1 = h;
+                    int i = 0;
+#pragma unroll 4
+                    for (; i + 1 < Ns; i += 2) {
+                        two_sum_acc(h, l, term(i, i * LS));
+                        two_sum_acc(h1, l1, term(i + 1, (i + 1) * LS));
+                    }
+                    if (i < Ns) two_sum_acc(h, l, term(i, i * LS));
+                    two_sum_acc(h, l, h1);
+                    l = fadd2(l, l1);
+                }
+#pragma unroll 1
+                for (int k0 = 0; k0 < L; k0 += 4) {
+                    float2 add[4], sub[4];
+#pragma unroll
+                    for (int v = 0; v < 4; ++v) {
+                        // the last row's step is not used
+                        const int i = min(k0 + v, max(L - 2, 0)), j = L > 1 ? i + Ns : 0;
+                        add[v] = term(j, rowq[j]);
+                        sub[v] = term(i, rowq[i]);
+                    }
+#pragma unroll
+                    for (int v = 0; v < 4; ++v) {
+                        float2 r = fadd2(h, l);
+                        if (FB) r = cscale(r, 0.5f);
+                        if (k0 + v < n) *out = r;
+                        out += (L - k0 - v + 1) & ~1;
+                        two_sum_acc(h, l, add[v]);
+                        two_sum_acc(h, l, make_float2(-sub[v].x, -sub[v].y));
+                    }
                 }
             }
         }
@@ -319,14 +389,22 @@ __global__ void general_format_r_kernel(long long n, int L, float scale, int ref
     }
 }
 
+// With few snapshots for the subarray length R is close to singular but for the
+// loading, and the rounding of the FP32 products, the same along a diagonal, shows
+// in P (L = 34, M = 65, K = 0: more than 1.5 times as far from 64 bits as with
+// exact products; at 2.5 L snapshots and more no difference).  Those frames take
+// the exact form.
+bool exact_form(const FrameDev &f) { return 2 * (2 * f.K + 1) * (f.M - f.L + 1) < 5 * f.L; }
+
 // the tile of a frame: two CTAs an SM where four pixels or more fit so, one
 // otherwise; no longer than what leaves every SM a unit.  tile 0: none fits.
 CovShape cov_shape(const FrameDev &f, int num_sms)
 {
     const int T = 2 * f.K + 1;
-    const CovShape one(1, f.K, f.M, f.L);
-    if (one.total > 226 * 1024) return CovShape(0, f.K, f.M, f.L);
-    const size_t per = ((size_t)one.XS + (size_t)one.QS) * sizeof(float2);
+    const bool exact = exact_form(f);
+    const CovShape one(1, f.K, f.M, f.L, exact);
+    if (one.total > 226 * 1024) return CovShape(0, f.K, f.M, f.L, exact);
+    const size_t per = (size_t)one.XS * sizeof(float2) + (size_t)one.QS * one.EB;
     auto room = [&](size_t most) {
         return one.total > most ? 0 : 1 + (int)std::min<size_t>(63, (most - one.total) / per);
     };
@@ -336,7 +414,7 @@ CovShape cov_shape(const FrameDev &f, int num_sms)
     tile = (int)std::min<long long>(std::min(tile, f.Npy), std::max<long long>(1, npix / num_sms));
     // whole passes of the diagonals' threads
     if (const int waves = tile * f.L / kCovThreads) tile = std::min(tile, waves * kCovThreads / f.L);
-    CovShape S(tile, f.K, f.M, f.L);
+    CovShape S(tile, f.K, f.M, f.L, exact);
     // product items along the tile: the count that keeps the threads fullest
     long best = -1;
     for (int ns = 1; tile && ns <= tile; ++ns) {
@@ -354,9 +432,10 @@ CovShape cov_shape(const FrameDev &f, int num_sms)
 }
 
 template <bool FB>
-auto cov_pick(int T)
+auto cov_pick(int T, bool exact)
 {
-    return T == 1   ? cov_kernel<1, FB>
+    return exact    ? cov_kernel<0, FB, true>
+           : T == 1   ? cov_kernel<1, FB>
            : T == 3 ? cov_kernel<3, FB>
            : T == 5 ? cov_kernel<5, FB>
            : T == 7 ? cov_kernel<7, FB>
@@ -365,15 +444,10 @@ auto cov_pick(int T)
 
 }  // namespace
 
-// With few subarrays the FP32 window products no longer average out of R (at
-// Ns = 6, L = 24, K = 2 P is 1.6 times as far from 64 bits as with exact
-// products); those frames stay with the precise pipeline.
-constexpr int kMinSubarrays = 12;
-
 bool general_supported(const FrameDev &f)
 {
-    if (f.L > 64 || f.refine || f.M - f.L + 1 < kMinSubarrays) return false;
-    const CovShape S(1, f.K, f.M, f.L);
+    if (f.L > 64 || f.refine) return false;
+    const CovShape S(1, f.K, f.M, f.L, exact_form(f));
     return S.total <= 226 * 1024 && f.M <= kCovMaxM;
 }
 
@@ -385,7 +459,8 @@ int launch_general(const FrameDev &f, float2 *work, unsigned *status, int num_sm
     if (S.tile < 1) return cudaErrorNotSupported;
     const long long units = (long long)f.Nx * ((f.Npy + S.tile - 1) / S.tile);
     if (units > 0x7fffffffLL - 65536) return cudaErrorInvalidValue;
-    auto kern = f.fb ? cov_pick<true>(2 * f.K + 1) : cov_pick<false>(2 * f.K + 1);
+    const bool exact = exact_form(f);
+    auto kern = f.fb ? cov_pick<true>(2 * f.K + 1, exact) : cov_pick<false>(2 * f.K + 1, exact);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S.total);
     if (e != cudaSuccess) return e;
     int per_sm = 0;

@@ -1,7 +1,7 @@
 // Precise element-space pipeline for sm_103a: the refinement option of the frames
-// without a fused instantiation, frames with few subarrays or a very wide
-// aperture (the general path of capon_general.cu takes the others), and the solve
-// stage of the tensor-core covariance forms.
+// without a fused instantiation, frames with a very wide aperture (the general path
+// of capon_general.cu takes the others), and the solve stage of the tensor-core
+// covariance forms.
 //
 //   1. covariance per pixel in float-float: along each diagonal d,
 //        R[k,k+d] = R0[d] + S[k,k+d],  S[k,k+d] = S[k-1,k-1+d] + D[k,k+d],

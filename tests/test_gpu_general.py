@@ -1,5 +1,5 @@
 """The general element-space path (subarray lengths without a fused kernel, long windows, forward-backward averaging;
-with fewer than 12 subarrays the precise pipeline): both sides of every padded length of its solve stage, windows with and without a compile-time row ring, odd channel
+exact products below 2.5 L snapshots): both sides of every padded length of its solve stage, windows with and without a compile-time row ring, odd channel
 counts, partial tiles, L = M and one pixel, against the FP64 oracle at the fused bars (P 1e-4, z 1e-3 of sqrt(P),
 w 2e-3; R to 1e-6 of its largest entry)."""
 import numpy as np
