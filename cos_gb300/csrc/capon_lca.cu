@@ -15,7 +15,8 @@
 // sums through the filter (FP32, yy then xx), a tap being one weight and one or
 // two 16-byte loads for all W windows.  What bounds it: issue, about 15
 // instructions a tap, then the read of Z; a [2048][256] image with 8 windows and a
-// 5 x 1 filter takes 18 us (2.2 TB/s over Z once and the outputs).  As two passes
+// 5 x 1 filter takes 16 us (2.4 TB/s over Z once and the outputs; 18 us with two CTAs
+// an SM instead of three).  As two passes
 // over memory, the planes |Z|^2 in HBM between them, it took 60 us; with a scalar
 // load, a multiply-add and the index arithmetic for every tap and window, 55 us.
 #include <algorithm>
@@ -31,7 +32,7 @@ static constexpr int kLcaTX = 32, kLcaTY = 16, kLcaThreads = 512;
 // W: windows a pixel holds in shared memory, S: its stride there in floats (8
 // lanes of a 16-byte load fall on all 32 banks: 4 and 12)
 template <int W>
-__global__ void __launch_bounds__(kLcaThreads, 2) lca_kernel(LcaDev a)
+__global__ void __launch_bounds__(kLcaThreads, 3) lca_kernel(LcaDev a)
 {
     constexpr int S = W == 4 ? 4 : 12;
     extern __shared__ __align__(16) float pw[];
