@@ -176,18 +176,22 @@ COS_DEV void async_copy8(void *dst, const void *src, bool is)
                  : "memory");
 }
 
+// window rows t0 .. t0+T-1 (T <= 32, a lane each); a longer window, or one whose
+// accumulators leave fewer than two CTAs an SM, takes several launches (backward pass
+// at M=128, L=32, K=4, [64][520]: 840 -> 640 us; M=33, L=16, K=17: 444 -> 354 us, both against
+// register-blocked tiles)
 template <int L, int SB>
-__global__ void __launch_bounds__(32 * kRowWarps, 2) adjoint_row_kernel(AdjDev a)
+__global__ void __launch_bounds__(32 * kRowWarps, 2) adjoint_row_kernel(AdjDev a, int t0, int T)
 {
     static_assert(SB % 2 == 0 && L % 2 == 0, "channel pairs are 16 bytes");
     extern __shared__ __align__(16) unsigned char smraw[];
-    const int M = a.M, T = 2 * a.K + 1, Ns = M - L + 1;
+    const int M = a.M, Ns = M - L + 1;
     const AdjRowSmem S(M, L, T, SB);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned char *const mine = smraw + warp * S.per_warp;
     float2 *const acc = (float2 *)(mine + S.off_a);
     float *const ths = (float *)(smraw + kRowWarps * S.per_warp) + (size_t)warp * M;   // channel-phase sums
-    const float scale = 1.0f / ((float)Ns * (float)T);
+    const float scale = 1.0f / ((float)Ns * (float)(2 * a.K + 1));
     const int nsb = (Ns + SB - 1) / SB, items = T * nsb;
     float dacc = 0.f;
     for (int c = lane; c < M; c += 32) ths[c] = 0.f;
@@ -197,9 +201,9 @@ __global__ void __launch_bounds__(32 * kRowWarps, 2) adjoint_row_kernel(AdjDev a
             ((float2 *)(mine + S.off_w))[(b * (T + 1) + T) * S.ws + l] = make_float2(0.f, 0.f);
     }
     const long long rows = (long long)a.Nx * a.Ny, step = (long long)gridDim.x * kRowWarps;
-    // gradient of pixel y-t on lane t (T <= 32); 0 where there is none
+    // gradient of pixel y-t0-t on lane t; 0 where there is none
     auto grad = [&](long long row) {
-        const int bx = (int)(row / a.Ny), p = (int)(row % a.Ny) - lane;
+        const int bx = (int)(row / a.Ny), p = (int)(row % a.Ny) - t0 - lane;
         return row < rows && lane < T && p >= 0 && p < a.Npy ? a.gP[(size_t)bx * a.Npy + p] : 0.f;
     };
     // the row's samples and the weights of its pixels (zeros where there is none)
@@ -210,7 +214,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 2) adjoint_row_kernel(AdjDev a
         const float2 *xr = a.x + (size_t)row * M;
         for (int c = lane; c < M; c += 32) async_copy8(xd + c, xr + c, true);
         for (int i = lane; i < T * L; i += 32) {
-            const int t = i / L, l = i % L, p = y - t;
+            const int t = i / L, l = i % L, p = y - t0 - t;
             const bool is = p >= 0 && p < a.Npy;
             async_copy8(wd + t * S.ws + l, a.w + ((size_t)bx * a.Npy + (is ? p : 0)) * L + l, is);
         }
@@ -247,7 +251,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 2) adjoint_row_kernel(AdjDev a
                 w[l] = make_float2(v.x, v.y);
                 w[l + 1] = make_float2(v.z, v.w);
             }
-            if (it < nsb) {   // t = 0: pixel y; one lane adds g |w|^2
+            if (t0 == 0 && it < nsb) {   // pixel y; one lane adds g |w|^2
                 float wn = 0.f;
 #pragma unroll
                 for (int l = 0; l < L; ++l) wn += cabs2(w[l]);
@@ -330,8 +334,9 @@ __global__ void __launch_bounds__(32 * kRowWarps, 2) adjoint_row_kernel(AdjDev a
     }
 }
 
-template <class Kern>
-static int launch_adjoint_with(Kern kern, const AdjDev &a, long long units, size_t smem, int num_sms, cudaStream_t s)
+template <class Kern, class... Args>
+static int launch_adjoint_with(Kern kern, const AdjDev &a, long long units, size_t smem, int num_sms, cudaStream_t s,
+                               Args... args)
 {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -340,29 +345,46 @@ static int launch_adjoint_with(Kern kern, const AdjDev &a, long long units, size
     if (e != cudaSuccess) return e;
     long long grid = (long long)num_sms * (per_sm > 0 ? per_sm : 1);
     if (grid > units) grid = units;
-    kern<<<(unsigned)grid, 32 * kAdjWarps, smem, s>>>(a);
+    kern<<<(unsigned)grid, 32 * kAdjWarps, smem, s>>>(a, args...);
     return cudaGetLastError();
+}
+
+// window rows a launch of the row kernel takes: at most 32 (a lane each) and what
+// leaves two CTAs an SM, spread evenly over the launches; the gradient rows add up.
+// 0: not even one row fits so
+static int rows_per_launch(const AdjDev &a)
+{
+    const int T = 2 * a.K + 1;
+    int most = T < 32 ? T : 32;
+    while (most > 0 && AdjRowSmem(a.M, a.L, most, 8).total > 112 * 1024) --most;
+    if (most == 0) return 0;
+    const int launches = (T + most - 1) / most;
+    return (T + launches - 1) / launches;
 }
 
 // SB: the block length that keeps the lanes fullest, passes of 32 items by the
 // products of an item
 template <int L>
-static int launch_rows(const AdjDev &a, int num_sms, cudaStream_t s)
+static int launch_rows(const AdjDev &a, int per, int num_sms, cudaStream_t s)
 {
     static_assert(kRowWarps == kAdjWarps, "one launch helper");
     const int T = 2 * a.K + 1, Ns = a.M - L + 1;
     const long long units = ((long long)a.Nx * a.Ny + kRowWarps - 1) / kRowWarps;
-    auto cost = [&](int sb) { return (T * ((Ns + sb - 1) / sb) + 31) / 32 * (sb + 2); };
-    auto go = [&](auto kern, int sb) {
-        return launch_adjoint_with(kern, a, units, AdjRowSmem(a.M, L, T, sb).total, num_sms, s);
-    };
+    auto cost = [&](int sb) { return (per * ((Ns + sb - 1) / sb) + 31) / 32 * (sb + 2); };
     int best = 2;
     for (int sb : {4, 6, 8})
         if (cost(sb) < cost(best)) best = sb;
-    return best == 2   ? go(adjoint_row_kernel<L, 2>, 2)
-           : best == 4 ? go(adjoint_row_kernel<L, 4>, 4)
-           : best == 6 ? go(adjoint_row_kernel<L, 6>, 6)
-                       : go(adjoint_row_kernel<L, 8>, 8);
+    for (int t0 = 0; t0 < T; t0 += per) {
+        const int n = T - t0 < per ? T - t0 : per;
+        const size_t smem = AdjRowSmem(a.M, L, n, best).total;
+        auto go = [&](auto kern) { return launch_adjoint_with(kern, a, units, smem, num_sms, s, t0, n); };
+        const int e = best == 2   ? go(adjoint_row_kernel<L, 2>)
+                      : best == 4 ? go(adjoint_row_kernel<L, 4>)
+                      : best == 6 ? go(adjoint_row_kernel<L, 6>)
+                                  : go(adjoint_row_kernel<L, 8>);
+        if (e) return e;
+    }
+    return 0;
 }
 
 int launch_adjoint(const AdjDev &a, int num_sms, cudaStream_t s)
@@ -371,14 +393,13 @@ int launch_adjoint(const AdjDev &a, int num_sms, cudaStream_t s)
     const size_t smem = (size_t)2 * rows * a.M * sizeof(float2) + (size_t)((a.M + 1) & ~1) * sizeof(float) +
                         (size_t)kAdjWarps * (a.L + T * Ns) * sizeof(float2);
     if (smem > 227 * 1024 || a.L > 64) return cudaErrorNotSupported;
-    // rows where they leave two CTAs an SM; the tiles serve the other lengths,
-    // very long windows and very wide apertures
-    if (T <= 32 && AdjRowSmem(a.M, a.L, T, 8).total <= 112 * 1024) {
+    // by rows; the tiles serve the other subarray lengths
+    if (const int per = rows_per_launch(a)) {
         switch (a.L) {
-        case 8: return launch_rows<8>(a, num_sms, s);
-        case 16: return launch_rows<16>(a, num_sms, s);
-        case 24: return launch_rows<24>(a, num_sms, s);
-        case 32: return launch_rows<32>(a, num_sms, s);
+        case 8: return launch_rows<8>(a, per, num_sms, s);
+        case 16: return launch_rows<16>(a, per, num_sms, s);
+        case 24: return launch_rows<24>(a, per, num_sms, s);
+        case 32: return launch_rows<32>(a, per, num_sms, s);
         default: break;
         }
     }

@@ -1,5 +1,5 @@
 """The row-wise adjoint at the edges of its lane blocks: one subarray, blocks that do not divide the subarrays, more
-items than lanes (several passes), long windows against few rows, masked gradients, against FP64 torch.linalg autograd.
+items than lanes (several passes), long windows against few rows and in several launches, masked gradients, against FP64 torch.linalg autograd.
 FP32 weights of a system of condition number up to about 1e3 carry about 1e-4; the bound is the adjoint's 1e-3."""
 import numpy as np
 import pytest
@@ -8,7 +8,8 @@ pytestmark = pytest.mark.gpu
 
 # L, K, M, Ny, Nx
 CASES = [(8, 0, 8, 5, 2), (8, 1, 21, 40, 3), (16, 3, 33, 20, 2), (16, 1, 32, 65, 2), (24, 2, 49, 33, 2), (24, 0, 71, 9, 1),
-         (32, 2, 64, 40, 2), (32, 1, 67, 31, 2), (32, 4, 33, 10, 1), (32, 0, 32, 3, 1), (20, 1, 40, 40, 2)]
+         (32, 2, 64, 40, 2), (32, 1, 67, 31, 2), (32, 4, 33, 10, 1), (32, 0, 32, 3, 1), (20, 1, 40, 40, 2),
+         (32, 4, 128, 30, 2), (16, 17, 33, 60, 1), (32, 9, 64, 40, 1)]
 
 
 @pytest.mark.parametrize("masked", [False, True])
