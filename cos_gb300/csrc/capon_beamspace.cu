@@ -246,6 +246,43 @@ beamspace_kernel(FrameDev f, float2 *__restrict__ Rbs)
     }
 }
 
+// The refinement's residual a_bs - (R + dl I) x in float-float: products exact by
+// fma, sums by TwoSum.  In FP64, at 2 multiply-adds a cycle and SM, it was the longest part
+// of a tile's solve: Nb = 3 and 5 in the four uneven frames of [256][1024] pixels
+// 1.94 -> 1.82 ms with outputs equal to 5e-10, Nb = 8 (M=64, L=32, K=1, 65 k pixels)
+// 257 -> 190 us together with tiles of 32 pixels instead of 16.
+// (h, l) += a x with a = (hi.re, hi.im, lo.re, lo.im): the high part's products
+// exact (TwoProd by fma), the low part's in FP32
+COS_DEV void bs_ff_cmac(float2 &h, float2 &l, float4 a, float2 x)
+{
+    const float2 xb = make_float2(-x.y, x.x);
+    const float2 sx = make_float2(a.x, a.x), sy = make_float2(a.y, a.y);
+    const float2 z = make_float2(0.f, 0.f);
+    const float2 p1 = ffma2(sx, x, z), p2 = ffma2(sy, xb, z);
+    const float2 e1 = ffma2(sx, x, make_float2(-p1.x, -p1.y)), e2 = ffma2(sy, xb, make_float2(-p2.x, -p2.y));
+    two_sum_acc(h, l, p1);
+    two_sum_acc(h, l, p2);
+    l = fadd2(l, fadd2(e1, e2));
+    l = ffma2(make_float2(a.z, a.z), x, l);
+    l = ffma2(make_float2(a.w, a.w), xb, l);
+}
+
+// the same with a real, exact a = d
+COS_DEV void bs_ff_rmac(float2 &h, float2 &l, float d, float2 x)
+{
+    const float2 s = make_float2(d, d), p = ffma2(s, x, make_float2(0.f, 0.f));
+    two_sum_acc(h, l, p);
+    l = fadd2(l, ffma2(s, x, make_float2(-p.x, -p.y)));
+}
+
+// a - (h + l)
+COS_DEV float2 bs_ff_residual(float2 a, float2 h, float2 l)
+{
+    float2 e = make_float2(0.f, 0.f);
+    two_sum_acc(a, e, make_float2(-h.x, -h.y));
+    return fadd2(a, fsub2(e, l));
+}
+
 // ---------------------------------------------------------------------------
 // Range-tile kernel for small beam counts (Nb <= 5).  A range row's subarray
 // DFTs are shared by the 2K+1 pixels whose window contains the row, so they
@@ -567,37 +604,24 @@ beamspace_tile_kernel(FrameDev f, float2 *__restrict__ Rbs, int tile)
 #pragma unroll
         for (int i = 0; i < NB; ++i) xb[i] = ab[i];
         solve(xb);
-        // FP64 residual against the float-float matrix, one correction
+        // residual against the float-float matrix, exact products in float-float;
+        // one correction
 #pragma unroll
         for (int i = 0; i < NB; ++i) {
-            double rr = (double)ab[i].x, ri = (double)ab[i].y;
+            float2 h = make_float2(0.f, 0.f), l = h;
 #pragma unroll
             for (int j = 0; j < NB; ++j) {
-                double ar, ai;
-                if (i <= j) {
-                    const int k = idx(i, j);
-                    ar = (double)Rh[k].x + (double)Rl[k].x;
-                    ai = (double)Rh[k].y + (double)Rl[k].y;
-                    if (loadVV) {
-                        ar += (double)dl * (double)VV[k].x;
-                        ai += (double)dl * (double)VV[k].y;
-                    } else if (i == j) {
-                        ar += (double)dl;
-                    }
-                    if (i == j) ai = 0.0;
-                } else {
-                    const int k = idx(j, i);
-                    ar = (double)Rh[k].x + (double)Rl[k].x;
-                    ai = -((double)Rh[k].y + (double)Rl[k].y);
-                    if (loadVV) {
-                        ar += (double)dl * (double)VV[k].x;
-                        ai -= (double)dl * (double)VV[k].y;
-                    }
+                const int k = i <= j ? idx(i, j) : idx(j, i);
+                auto im = [&](float y) { return i < j ? y : i > j ? -y : 0.f; };   // left of the diagonal: conjugates
+                bs_ff_cmac(h, l, make_float4(Rh[k].x, im(Rh[k].y), Rl[k].x, im(Rl[k].y)), xb[j]);
+                if (loadVV) {
+                    const float2 v = make_float2(VV[k].x, im(VV[k].y)), d2 = make_float2(dl, dl);
+                    const float2 q = ffma2(d2, v, make_float2(0.f, 0.f)), e = ffma2(d2, v, make_float2(-q.x, -q.y));
+                    bs_ff_cmac(h, l, make_float4(q.x, q.y, e.x, e.y), xb[j]);
                 }
-                rr -= ar * (double)xb[j].x - ai * (double)xb[j].y;
-                ri -= ar * (double)xb[j].y + ai * (double)xb[j].x;
             }
-            r[i] = make_float2((float)rr, (float)ri);
+            if (!loadVV) bs_ff_rmac(h, l, dl, xb[i]);
+            r[i] = bs_ff_residual(ab[i], h, l);
         }
         solve(r);
         float2 aRa = make_float2(0.f, 0.f), zn = make_float2(0.f, 0.f);
@@ -653,8 +677,8 @@ static int launch_tile(const FrameDev &f, float2 *R_out, cudaStream_t s)
 //
 // The warp kernel above redoes the DFT and the products of every window row
 // for every pixel and leaves the Nb x Nb solve to one lane; at M=64, L=32,
-// K=1, Nb=8 with weights it needs 3.90 ms for 65 k pixels, this kernel 0.26 ms
-// (13 GB/s -> 196 GB/s of the frame's own bytes).  Here a CTA owns a
+// K=1, Nb=8 with weights it needs 3.90 ms for 65 k pixels, this kernel 0.19 ms
+// (13 GB/s -> 265 GB/s of the frame's own bytes).  Here a CTA owns a
 // run of pixels of one beam and does each row's work once:
 //   rows    Y[row][s][b] by the sliding DFT in chunks of kWideChunk subarrays
 //           (direct at the chunk start), the row's energy sum_m c_m |x_m|^2
@@ -687,13 +711,15 @@ struct BsWideSmem {
         auto up = [](size_t v) { return (v + 15) & ~(size_t)15; };
         off_b = 0;                                                        // Butler L x NbE, rot, a_bs
         off_x = off_b + up((size_t)(L * NbE + 2 * NbE) * sizeof(float2));
-        off_e = off_x + up((size_t)rows * M * sizeof(float2));
+        // tile x (Nb + 1), once the samples have been read; beside them, it left room
+        // for 16 pixels only in the case timed above
+        off_xb = off_x;
+        off_e = off_x + up((size_t)(rows * M > tile * (Nb + 1) ? rows * M : tile * (Nb + 1)) * sizeof(float2));
         off_g = off_e + up((size_t)rows * sizeof(float));
         off_q = off_g + up((size_t)rows * NbE * sizeof(float2));          // rows x NQ (hi, lo)
-        off_xb = off_q + up((size_t)rows * NQ * sizeof(float4));          // tile x (Nb + 1)
+        off_y = off_q + up((size_t)rows * NQ * sizeof(float4));
         // Y is dead once the row products are formed: the pixels' matrices and
         // the solve's exchange rows take its place
-        off_y = off_xb + up((size_t)tile * (Nb + 1) * sizeof(float2));
         off_r = off_y;                                                    // tile x NQ (hi, lo)
         off_u = off_r + up((size_t)tile * NQ * sizeof(float4));           // (256 / G) x G x (G + 1)
         const size_t y_end = off_y + up((size_t)rows * Ns * NbE * sizeof(float2));
@@ -701,22 +727,6 @@ struct BsWideSmem {
         total = y_end > u_end ? y_end : u_end;
     }
 };
-
-// (h, l) += a x with a = (hi.re, hi.im, lo.re, lo.im): the high part's products
-// exact (TwoProd by fma), the low part's in FP32
-COS_DEV void bs_ff_cmac(float2 &h, float2 &l, float4 a, float2 x)
-{
-    const float2 xb = make_float2(-x.y, x.x);
-    const float2 sx = make_float2(a.x, a.x), sy = make_float2(a.y, a.y);
-    const float2 z = make_float2(0.f, 0.f);
-    const float2 p1 = ffma2(sx, x, z), p2 = ffma2(sy, xb, z);
-    const float2 e1 = ffma2(sx, x, make_float2(-p1.x, -p1.y)), e2 = ffma2(sy, xb, make_float2(-p2.x, -p2.y));
-    two_sum_acc(h, l, p1);
-    two_sum_acc(h, l, p2);
-    l = fadd2(l, fadd2(e1, e2));
-    l = ffma2(make_float2(a.z, a.z), x, l);
-    l = ffma2(make_float2(a.w, a.w), xb, l);
-}
 
 // i / d by the reciprocal of d; exact while the quotient times d stays below 2^21
 COS_DEV int bs_div(int i, float inv) { return (int)(((float)i + 0.5f) * inv); }
@@ -972,12 +982,8 @@ beamspace_wide_kernel(FrameDev f, float2 *__restrict__ Rbs, int tile, int units)
                         bs_ff_cmac(h, lo, e, xi);
                     }
                 }
-                float2 r;
-                {
-                    const double rre = ((double)a0.x - (double)dl * (double)x.x) - (double)h.x - (double)lo.x;
-                    const double rim = ((double)a0.y - (double)dl * (double)x.y) - (double)h.y - (double)lo.y;
-                    r = make_float2((float)rre, (float)rim);
-                }
+                bs_ff_rmac(h, lo, dl, x);
+                float2 r = bs_ff_residual(a0, h, lo);
                 // forward solve with the column the lane holds
     #pragma unroll
                 for (int i = 0; i < G; ++i) {
@@ -1072,7 +1078,7 @@ int launch_beamspace(const FrameDev &f, float2 *R_out, cudaStream_t s)
     default: break;
     }
     // the sizes served are the warp kernel's; within them the row-sharing
-    // kernel wherever a tile of it fits (3.90 -> 0.26 ms at M=64, L=32, K=1,
+    // kernel wherever a tile of it fits (3.90 -> 0.19 ms at M=64, L=32, K=1,
     // Nb=8), Nb > 32 and very long windows with one warp per pixel
     if (f.L > 64 || BsSmem(f.M, f.L, f.K, f.Nb).total > 227 * 1024) return cudaErrorNotSupported;
     if (f.Nb <= kWideMaxNb) {
