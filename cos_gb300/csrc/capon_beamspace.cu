@@ -680,8 +680,12 @@ static int launch_tile(const FrameDev &f, float2 *R_out, cudaStream_t s)
 // K=1, Nb=8 with weights it needs 3.90 ms for 65 k pixels, this kernel 0.19 ms
 // (13 GB/s -> 265 GB/s of the frame's own bytes).  Here a CTA owns a
 // run of pixels of one beam and does each row's work once:
-//   rows    Y[row][s][b] by the sliding DFT in chunks of kWideChunk subarrays
-//           (direct at the chunk start), the row's energy sum_m c_m |x_m|^2
+//   rows    Y[row][s][b] by the DFT: directly for every third subarray, its two
+//           neighbours by the sliding recurrence (a direct sum's rounding is
+//           shared by the three and adds up over them: as one running sum at the
+//           first of the three, the weights' error was up to twice the warp
+//           kernel's; as four sums in the middle it is 0.7 to 1.1 of it, in the
+//           same time.  Five from the middle's sum: 0.18 ms, but past it again), the row's energy sum_m c_m |x_m|^2
 //           (c_m: how many subarrays hold channel m) and the beam sums;
 //   Q_row   the Nb x Nb products in 2 x 2 blocks per thread, four terms in
 //           FP32, chunk sums in float-float;
@@ -695,7 +699,6 @@ static int launch_tile(const FrameDev &f, float2 *R_out, cudaStream_t s)
 // is the largest of 32, 16, 8 pixels that leaves two CTAs an SM to overlap
 // one's loads and barriers with the other's arithmetic.
 static constexpr int kWideThreads = 256;
-static constexpr int kWideChunk = 3;
 static constexpr int kWideMaxNb = 32;
 
 struct BsWideSmem {
@@ -792,28 +795,43 @@ beamspace_wide_kernel(FrameDev f, float2 *__restrict__ Rbs, int tile, int units)
 
         // ---- rows: the sliding DFT, two beams per thread
         {
-            const int nch = (Ns + kWideChunk - 1) / kWideChunk, nbp = NbE / 2;
+            const int nch = (Ns + 2) / 3, nbp = NbE / 2;
             const float inv_nbp = 1.f / (float)nbp, inv_nch = 1.f / (float)nch;
             for (int it = tid; it < rows * nch * nbp; it += kWideThreads) {
                 const int rc = bs_div(it, inv_nbp), b = 2 * (it - rc * nbp), r = bs_div(rc, inv_nch), ch = rc - r * nch;
-                const int s0 = ch * kWideChunk, s1 = min(Ns, s0 + kWideChunk);
-                const float2 *xr = xs + (size_t)r * M;
-                float2 y0 = make_float2(0.f, 0.f), y1 = make_float2(0.f, 0.f);
-                for (int l = 0; l < L; ++l) {
-                    const float2 v = xr[s0 + l];
+                // direct in the chunk's middle, one step of the recurrence either way
+                const int s0 = ch * 3, sc = min(s0 + 1, Ns - 1);
+                const float2 *xr = xs + (size_t)r * M + sc;
+                // four partial sums a beam: the chunk's subarrays share this sum's rounding
+                float2 q0[4], q1[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) q0[k] = q1[k] = make_float2(0.f, 0.f);
+                auto term = [&](int k, int l) {
+                    const float2 v = xr[l];
                     const float4 bb = *(const float4 *)(Bt + l * NbE + b);
-                    y0 = cmac4(y0, make_float2(bb.x, bb.y), v);
-                    y1 = cmac4(y1, make_float2(bb.z, bb.w), v);
+                    q0[k] = cmac4(q0[k], make_float2(bb.x, bb.y), v);
+                    q1[k] = cmac4(q1[k], make_float2(bb.z, bb.w), v);
+                };
+                int l = 0;
+                for (; l + 3 < L; l += 4) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) term(k, l + k);
                 }
+                for (; l < L; ++l) term(0, l);
+                const float2 y0 = fadd2(fadd2(q0[0], q0[1]), fadd2(q0[2], q0[3]));
+                const float2 y1 = fadd2(fadd2(q1[0], q1[1]), fadd2(q1[2], q1[3]));
                 const float2 r0 = rot[b], r1 = rot[b + 1];
-                float2 *yr = Y + ((size_t)r * Ns + s0) * NbE + b;
+                float2 *yr = Y + ((size_t)r * Ns + sc) * NbE + b;
                 *(float4 *)yr = make_float4(y0.x, y0.y, y1.x, y1.y);
-                for (int s = s0 + 1; s < s1; ++s) {
-                    yr += NbE;
-                    const float2 dx = cscale(csub(xr[s - 1 + L], xr[s - 1]), isl);
-                    y0 = cmul(r0, cadd(y0, dx));
-                    y1 = cmul(r1, cadd(y1, dx));
-                    *(float4 *)yr = make_float4(y0.x, y0.y, y1.x, y1.y);
+                if (sc + 1 < min(Ns, s0 + 3)) {
+                    const float2 dx = cscale(csub(xr[L], xr[0]), isl);
+                    const float2 u0 = cmul(r0, cadd(y0, dx)), u1 = cmul(r1, cadd(y1, dx));
+                    *(float4 *)(yr + NbE) = make_float4(u0.x, u0.y, u1.x, u1.y);
+                }
+                if (sc > s0) {
+                    const float2 dx = cscale(csub(xr[L - 1], xr[-1]), isl);
+                    const float2 u0 = csub(cconjmul(r0, y0), dx), u1 = csub(cconjmul(r1, y1), dx);
+                    *(float4 *)(yr - NbE) = make_float4(u0.x, u0.y, u1.x, u1.y);
                 }
             }
         }
