@@ -725,10 +725,11 @@ int cos_capon_tdib(cos_capon_ctx *c, const void *mfdata, int n_hydros, int n_sam
     TdibDev t;
     memset(&t, 0, sizeof(t));
     t.t0 = t0;
-    t.dt = dt;
     t.inv_dt = 1.0 / dt;
     t.inv_c = 1.0 / cs;
     t.fc = fc;
+    t.ku = (float)(t.inv_c / dt);
+    t.kc = (float)(fc * t.inv_c);
     t.n_hydros = n_hydros;
     t.n_samples = n_samples;
     t.n_x = n_x;

@@ -685,7 +685,8 @@ static int launch_tile(const FrameDev &f, float2 *R_out, cudaStream_t s)
 //           shared by the three and adds up over them: as one running sum at the
 //           first of the three, the weights' error was up to twice the warp
 //           kernel's; as four sums in the middle it is 0.7 to 1.1 of it, in the
-//           same time.  Five from the middle's sum: 0.18 ms, but past it again), the row's energy sum_m c_m |x_m|^2
+//           same time; five from the first: 0.18 ms, up to 2.3 times), the row's
+//           energy sum_m c_m |x_m|^2
 //           (c_m: how many subarrays hold channel m) and the beam sums;
 //   Q_row   the Nb x Nb products in 2 x 2 blocks per thread, four terms in
 //           FP32, chunk sums in float-float;
