@@ -7,7 +7,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("N", [1, 2, 7, 8, 9, 15, 16, 17, 24, 25, 31, 32, 33, 47, 48, 49, 63, 64, 65, 71, 72])
+@pytest.mark.parametrize("N", [1, 2, 7, 8, 9, 15, 16, 17, 24, 25, 31, 32, 33, 36, 37, 40, 41, 47, 48, 49, 63, 64, 65, 71, 72])
 def test_lu_sizes(N):
     from cos_gb300 import capon
     rng = np.random.default_rng(N)
