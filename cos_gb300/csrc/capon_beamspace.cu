@@ -959,6 +959,7 @@ beamspace_wide_kernel(FrameDev f, float2 *__restrict__ Rbs, int tile, int units)
                 const float2 a0 = c >= 0 ? ab[c] : make_float2(0.f, 0.f);
                 float2 y = a0;         // L^-1 a_bs, row j
                 float dinv = 1.f;      // 1 / d_j
+                bool bad = false;      // a pivot that is not positive, the same for all lanes of the pixel
                 // step i: row i of the factor in X[i], then the rows below
                 __syncwarp();
     #pragma unroll
@@ -967,7 +968,9 @@ beamspace_wide_kernel(FrameDev f, float2 *__restrict__ Rbs, int tile, int units)
                     X[i * (G + 1) + j] = A[i];
                     if (j == i) X[i * (G + 1) + G] = y;
                     __syncwarp();
-                    const float rd = __frcp_rn(X[i * (G + 1) + i].x);
+                    const float dv = X[i * (G + 1) + i].x;
+                    bad |= !(dv > 0.f);
+                    const float rd = __frcp_rn(dv);
                     const float2 yi = cscale(X[i * (G + 1) + G], rd);
                     if (j == i) dinv = rd;
                     if (j > i) {
@@ -1011,6 +1014,8 @@ beamspace_wide_kernel(FrameDev f, float2 *__restrict__ Rbs, int tile, int units)
                     if (j > i) r = csub(r, cconjmul(A[i], ri));
                 }
                 x = cadd(x, back(r));
+                // no Cholesky factor: outputs not finite, as a square root of the pivot would leave them
+                if (bad) x = make_float2(__int_as_float(0x7fc00000), __int_as_float(0x7fc00000));
                 // sum(Ria) = a_bs^H x; z = conj(x)^T g_bs / conj(sum), g_bs = beam sums / Ns
                 float2 aRa = make_float2(0.f, 0.f), zn = aRa;
                 if (c >= 0) {
