@@ -9,9 +9,15 @@
 // factorisations, since a warp's triangle leaves no room to load ahead.
 //
 // G lanes own one pixel, lane r the columns j = m*G + r of the upper triangle
-// (m < LP/G).  The factorisation is that of the fused kernels (R = L D L^H,
-// matrixDecompc.pyx:19-50, the right-hand sides carried along), with the
-// pivot row broadcast through shared memory.  A subarray length between two
+// (m < LP/G).  R = U^H U (matrixDecompc.pyx:19-50), the right-hand sides carried
+// along, a row scaled by its pivot's inverse square root and broadcast through shared
+// memory; a product is formed and then subtracted.  The fused kernels' form, R =
+// L D L^H with the product subtracted by two fmas, is faster (65 k pixels, L = 32, z
+// and P: 0.17 ms, 0.19 so; 60 k pixels, L = 24, weights: 0.13 and 0.15) but rounds
+// twice at the entry's size, and its update carries the rounding of the multipliers,
+// which a factor used on both sides does not: w was 1.1 to 1.27 times as far from 64
+// bits as in the precise pipeline at L = 33 to 64 (P up to 1.19 times), 0.95 to 1.01
+// times so.  A subarray length between two
 // instantiations is padded in front: rows and columns 0 .. pad-1 (pad = LP - L)
 // are an identity with zero right-hand sides, and the unrolled steps of those
 // rows are skipped, so that padding costs idle column slots only -- the steps
@@ -72,6 +78,7 @@ solve_kernel(FrameDev f, const float2 *__restrict__ work, long long npix, unsign
     float2 *const in = (float2 *)(smraw + C::BAR + (size_t)C::WARPS * PPW * C::AREA * sizeof(float4)) +
                        (size_t)warp * PPW * rec;
     const float nt = (float)(f.M - L + 1) * (float)(2 * f.K + 1);
+    const float2 zero = make_float2(0.f, 0.f);
     const long long step = (long long)gridDim.x * C::WARPS * PPW;
     long long p0 = ((long long)blockIdx.x * C::WARPS + warp) * PPW;
     // lane 0: the records of pixels p .. p+PPW-1 (the last one again past the end)
@@ -132,15 +139,26 @@ solve_kernel(FrameDev f, const float2 *__restrict__ work, long long npix, unsign
         bool bad = false;
         float s11 = 0.f, s11l = 0.f;  // high part and the sum of its rounding errors
         float2 s12 = make_float2(0.f, 0.f);
-        // row `row` as (-Re, +Im, -Im, -Re) of A[row][j]; slot LP carries the
-        // row's right-hand sides
+        // row `row` and its right-hand sides by the pivot's inverse square root, then
+        // the row as (-Re, +Im, -Im, -Re) of U[row][j]; slot LP carries the right-hand sides
         auto publish = [&](auto rc, float4 *buf) __attribute__((always_inline)) {
             constexpr int row = decltype(rc)::value, mrow = row / G;
+            const float dv = __shfl_sync(0xffffffffu, A[row][mrow].x, row % G, G);
+            bad |= !(dv > 0.f);
+            // the unit's approximation and one Newton step: its error is common to the
+            // whole row
+            const float y0 = rsqrtf(dv), inv = fmaf(0.5f * y0, fmaf(-dv * y0, y0, 1.f), y0);
 #pragma unroll
-            for (int m = mrow; m < NM; ++m)
+            for (int m = mrow; m < NM; ++m) {
+                A[row][m] = cscale(A[row][m], inv);
                 buf[m * G + r] = make_float4(-A[row][m].x, A[row][m].y, -A[row][m].y, -A[row][m].x);
-            if (r == row % G)
+            }
+            if (r == row % G) {
+                if (W) dinv[mrow] = inv;
+                b1[mrow] = cscale(b1[mrow], inv);
+                if (!W) b2[mrow] = cscale(b2[mrow], inv);
                 buf[LP] = make_float4(b1[mrow].x, b1[mrow].y, W ? 0.f : b2[mrow].x, W ? 0.f : b2[mrow].y);
+            }
         };
         __syncwarp();  // the area's readers of the last pixel are done
         if (pad == 0) publish(std::integral_constant<int, 0>{}, rb);
@@ -156,34 +174,29 @@ solve_kernel(FrameDev f, const float2 *__restrict__ work, long long npix, unsign
                 // at step i-2, before the barrier that ended step i-1
                 float4 *const rbi = rb + (i & 1) * (LP + 1);
                 __syncwarp();
-                const float dv = -rbi[i].x;
                 const float4 yy = rbi[LP];
-                bad |= !(dv > 0.f);
-                const float rdv = __frcp_rn(dv);
-                if (W && r == oi) dinv[mi] = rdv;
-                const float2 y1 = make_float2(yy.x * rdv, yy.y * rdv), y2 = make_float2(yy.z * rdv, yy.w * rdv);
+                const float2 y1 = make_float2(yy.x, yy.y), y2 = make_float2(yy.z, yy.w);
                 {
-                    const float t = fmaf(yy.x, y1.x, yy.y * y1.y), s = s11 + t;
+                    const float t = cabs2(y1), s = s11 + t;
                     s11l += t - (s - s11);
                     s11 = s;
                 }
-                if (!W) s12 = cadd(s12, cconjmul(make_float2(yy.x, yy.y), y2));
+                if (!W) s12 = cadd(s12, cconjmul(y1, y2));
                 const float2 y1s = make_float2(y1.y, y1.x), y2s = make_float2(y2.y, y2.x);
                 float2 vrr[NM], vii[NM];
 #pragma unroll
                 for (int m = mi; m < NM; ++m) {
                     const float2 v = A[i][m];
                     const float2 n1 = make_float2(-v.x, -v.x), n2 = make_float2(-v.y, v.y);
-                    const float2 t1 = ffma2(n2, y1s, ffma2(n1, y1, b1[m]));
+                    const float2 t1 = fadd2(b1[m], ffma2(n2, y1s, ffma2(n1, y1, zero)));
                     const bool below = m > mi || r > oi;
                     if (below) b1[m] = t1;
                     if (!W) {
-                        const float2 t2 = ffma2(n2, y2s, ffma2(n1, y2, b2[m]));
+                        const float2 t2 = fadd2(b2[m], ffma2(n2, y2s, ffma2(n1, y2, zero)));
                         if (below) b2[m] = t2;
                     }
-                    const float vr = v.x * rdv, vi = v.y * rdv;
-                    vrr[m] = make_float2(vr, vr);
-                    vii[m] = make_float2(vi, vi);
+                    vrr[m] = make_float2(v.x, v.x);
+                    vii[m] = make_float2(v.y, v.y);
                 }
                 // row i+1 first, published before the bulk of the update
 #pragma unroll
@@ -192,8 +205,8 @@ solve_kernel(FrameDev f, const float2 *__restrict__ work, long long npix, unsign
 #pragma unroll
                     for (int m = mi; m < NM; ++m)
                         if (m >= k / G)
-                            A[k][m] = ffma2(vii[m], make_float2(u4.z, u4.w),
-                                            ffma2(vrr[m], make_float2(u4.x, u4.y), A[k][m]));
+                            A[k][m] = fadd2(A[k][m], ffma2(vii[m], make_float2(u4.z, u4.w),
+                                                           ffma2(vrr[m], make_float2(u4.x, u4.y), zero)));
                     if constexpr (i + 1 < LP)
                         if (k == i + 1) publish(std::integral_constant<int, i + 1>{}, nxt);
                 }
@@ -208,7 +221,7 @@ solve_kernel(FrameDev f, const float2 *__restrict__ work, long long npix, unsign
             if (bad) atomicOr(status, ERR_NOT_PD);
         }
         if constexpr (W) {
-            // (D L^H) x = b1 by blocks of G rows, last block first, through the
+            // U x = b1 by blocks of G rows, last block first, through the
             // exchange area (the fused w mode's scheme, capon_fused.cuh)
             float2 xv[NM];
 #pragma unroll
