@@ -388,9 +388,11 @@ auto cov_pick(int T)
 
 }  // namespace
 
+// the sizes served are the precise pipeline's (its four warps' sample windows in
+// shared memory), within them whatever a tile of one pixel fits
 bool general_supported(const FrameDev &f)
 {
-    if (f.L > 64 || f.refine) return false;
+    if (f.L > 64 || f.refine || (size_t)4 * (2 * f.K + 1) * f.M * sizeof(float2) > 227 * 1024) return false;
     // the fewest pairs that cov_shape tries
     return CovShape(1, ((f.L + 1) / 2 + kCovParts - 1) / kCovParts, f.K, f.M, f.L).total <= 226 * 1024;
 }
