@@ -263,14 +263,6 @@ static int run_plain(cos_capon_ctx *c, FrameDev f, cudaStream_t s)
     return e;
 }
 
-// general path for one element-space frame: covariance rows, then the register
-// solve
-static int run_general(cos_capon_ctx *c, FrameDev f, cudaStream_t s)
-{
-    if (int e = c->Rwork.ensure(general_bytes(f))) return e;
-    return launch_general(f, (float2 *)c->Rwork.p, c->d_status, c->num_sms, s);
-}
-
 // precise pipeline (float-float covariance, FP32 Cholesky, optional FP64-residual
 // refinement) for one element-space frame
 static int run_precise(cos_capon_ctx *c, FrameDev f, bool refine, cudaStream_t s)
@@ -287,6 +279,15 @@ static int run_precise(cos_capon_ctx *c, FrameDev f, bool refine, cudaStream_t s
     // the requested R is the float-float matrix the solve used, plus the loading
     if (f.R) e = launch_format_r(f, (float2 *)c->Rwork.p, (float2 *)c->Rlo.p, (float *)c->dl.p, f.R, s);
     return e;
+}
+
+// general path for one element-space frame: covariance rows, then the register
+// solve.  Only at L = 1 does its record take more than the pipeline's buffers: where
+// that is too much, the pipeline
+static int run_general(cos_capon_ctx *c, FrameDev f, cudaStream_t s)
+{
+    if (c->Rwork.ensure(general_bytes(f))) return run_precise(c, f, false, s);
+    return launch_general(f, (float2 *)c->Rwork.p, c->d_status, c->num_sms, s);
 }
 
 static bool is_tc_form(int form)
@@ -310,6 +311,12 @@ static int run_tc(cos_capon_ctx *c, FrameDev f, int split, bool refine, cudaStre
     if ((e = launch_precise_solve(f, Rw, nullptr, dl, (float2 *)c->Ria.p, c->d_status, refine, s))) return e;
     if (f.R) e = launch_format_r(f, Rw, nullptr, dl, f.R, s);
     return e;
+}
+
+// an element-space frame without a fused instantiation that takes the general path
+static bool use_general(const FrameDev &f, const cos_capon_opts &o)
+{
+    return !is_tc_form(o.form) && (o.form != COS_CAPON_FORM_PLAIN || o.refine) && general_supported(f);
 }
 
 static int run_frames(cos_capon_ctx *c, const FrameDev *fs, int n, const cos_capon_opts &o, cudaStream_t s)
@@ -421,7 +428,7 @@ static int run_frames(cos_capon_ctx *c, const FrameDev *fs, int n, const cos_cap
         // pipeline; the plain form when asked for
         return is_tc_form(o.form)                              ? run_tc(c, f, o.form, o.refine != 0, st)
                : (o.form == COS_CAPON_FORM_PLAIN && !o.refine) ? run_plain(c, f, st)
-               : general_supported(f)                          ? run_general(c, f, st)
+               : use_general(f, o)                             ? run_general(c, f, st)
                                                                : run_precise(c, f, o.refine != 0, st);
     };
     // Groups that use no context scratch (fused, beamspace) may run side by
@@ -608,9 +615,16 @@ static int get_capon_host(cos_capon_ctx *c, void *z, float *P, void *w, void *R,
     need += (R && bR > c->R.cap) ? bR : 0;
     const bool sliding = o.form == COS_CAPON_FORM_SLIDING_INVERSE;
     if (plain && Nb == 0 && !sliding) {
-        const size_t br = std::max(bR, general_bytes(make_frame(whole, o)));   // more than R at the shortest L
-        need += (br > c->Rwork.cap ? br : 0) + (bw > c->Ria.cap ? bw : 0);
-        if (!(o.form == COS_CAPON_FORM_PLAIN && !o.refine)) need += bR > c->Rlo.cap ? bR : 0;
+        // the work buffers of run_plain, run_precise and run_tc, or the general path's
+        // records alone
+        size_t work = (bR > c->Rwork.cap ? bR : 0) + (bw > c->Ria.cap ? bw : 0);
+        if (!(o.form == COS_CAPON_FORM_PLAIN && !o.refine)) work += bR > c->Rlo.cap ? bR : 0;
+        const FrameDev f = make_frame(whole, o);
+        if (use_general(f, o)) {
+            const size_t br = general_bytes(f);
+            work = std::min(work, br > c->Rwork.cap ? br : 0);
+        }
+        need += work;
     }
     if ((e = check_free(need))) return e;
     if ((e = c->x.ensure(bx)) || (e = c->z.ensure(bz))) return e;
