@@ -739,7 +739,7 @@ int cos_capon_tdib(cos_capon_ctx *c, const void *mfdata, int n_hydros, int n_sam
     TdibDev t;
     memset(&t, 0, sizeof(t));
     t.t0 = t0;
-    t.inv_dt = 1.0 / dt;
+    t.dt = dt;
     t.inv_c = 1.0 / cs;
     t.fc = fc;
     t.ku = (float)(t.inv_c / dt);

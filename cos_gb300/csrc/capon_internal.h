@@ -157,7 +157,7 @@ struct TdibDev {
     const double *D;       // [n_hydros] receiver depths
     const double *xarr;    // [n_x][n_y] pixel x
     const double *yarr;    // [n_x][n_y] pixel y
-    double t0, inv_dt, inv_c, fc;
+    double t0, dt, inv_c, fc;
     float ku, kc;          // samples and carrier cycles a unit of path
     int n_hydros, n_samples, n_x, n_y;
     float2 *Xd;            // [n_x][n_y][n_hydros] or null

@@ -102,7 +102,8 @@ __global__ void __launch_bounds__(32 * kTdibWarps, 4) tdib_kernel(TdibDev t)
             const double X = t.xarr[(size_t)nx * t.n_y + yl], Y = t.yarr[(size_t)nx * t.n_y + yl];
             const double ax = xx + X, rt2 = ax * ax + Y * Y + zz * zz, rt = sqrt(rt2);
             const double tau0 = 2.0 * rt * t.inv_c;
-            const double u0 = (tau0 - t.t0) * t.inv_dt;
+            // a quotient: a delay on the last sample must not come out past it
+            const double u0 = (tau0 - t.t0) / t.dt;
             const double fu = floor(u0);
             const double cyc = t.fc * tau0;
             b = (int)fu;
