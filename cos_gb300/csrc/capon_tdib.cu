@@ -43,7 +43,7 @@ COS_DEV float quotient(float n, float d)
     return fmaf(y, fmaf(-q, d, n), q);
 }
 
-// A warp takes 32 consecutive range pixels of one beam, a pixel per lane.  The
+// A warp takes 32 consecutive pixels of the fan, beam after beam, a pixel per lane.  The
 // lane evaluates the FP64 part of its pixel once: r_t, the base delay 2 r_t / c
 // split into an integer sample index and a fraction, and the base carrier phase
 // fc 2 r_t / c reduced to a fraction of a cycle.  Per hydrophone only the small
@@ -56,51 +56,74 @@ COS_DEV float quotient(float n, float d)
 // The pixel sits on the lane, not the hydrophone, for the gathers: neighbouring
 // range pixels read neighbouring samples of one channel, a few cache lines a
 // load, where 32 channels are 32 lines (263 us for [256][2048] pixels x 64
-// hydrophones, bound by the line rate of L1; 158 us so, bound by
+// hydrophones, bound by the line rate of L1; 152 us so, bound by
 // issue, about 110 instructions an element).  Persistent CTAs, four an SM: the origin and
-// the hydrophones' terms, as much FP64 as a run of pixels itself, are formed once
-// a CTA (a CTA per 256 pixels: 164 us; three an SM at 75 registers 162 us,
-// five 193 us).  The cube's rows run over
+// the hydrophones' terms are formed once a CTA, the origin by one of its warps (by all
+// of them: 159 us).  (A CTA per 256 pixels is 4 % slower, three an SM at 75 registers 3 %,
+// five 22 %.)  The cube's rows run over
 // the hydrophones, so the samples of 16 of them pass through shared memory and
 // leave as whole 128-byte rows.
-__global__ void __launch_bounds__(32 * kTdibWarps, 4) tdib_kernel(TdibDev t)
+//
+// SPLIT, for calls that leave warps idle: `parts` warps of a CTA share 32 pixels, cw
+// hydrophones (4, 8 or 16) each in turn; the FP64 part is the first one's, and their
+// image sums meet in shared memory.  [8][1] pixels x 250 hydrophones: 25 us, 69 us by
+// one warp (26 us with a hydrophone per lane); [512][2] x 64: 18 us, 32 us (23 us).
+template <bool SPLIT>
+__global__ void __launch_bounds__(32 * kTdibWarps, 4) tdib_kernel(TdibDev t, int parts, int cw)
 {
+    if (!SPLIT) {
+        parts = 1;
+        cw = kTdibChunk;
+    }
     __shared__ float2 hyd[kTdibMaxHydros];                       // (x_n, c_n)
+    __shared__ double origin[2];
+    __shared__ float base[SPLIT ? kTdibWarps : 1][6][32];        // a group's FP64 results
+    __shared__ float2 part[SPLIT ? kTdibWarps : 1][32];          // image sums of the warps
     __shared__ float2 tile[kTdibWarps][32][kTdibChunk + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // origin: half the mean receiver position and depth (the same
-    // lane-strided sums and butterfly in every warp)
-    double sx = 0.0, sz = 0.0;
-    for (int n = lane; n < t.n_hydros; n += 32) {
-        sx += t.x_r[n];
-        sz += t.D[n];
+    // origin: half the mean receiver position and depth, by one warp (FP64 of all
+    // eight would take as long as a run of pixels)
+    if (warp == 0) {
+        double sx = 0.0, sz = 0.0;
+        for (int n = lane; n < t.n_hydros; n += 32) {
+            sx += t.x_r[n];
+            sz += t.D[n];
+        }
+        for (int o = 16; o; o >>= 1) {
+            sx += __shfl_xor_sync(0xffffffffu, sx, o);
+            sz += __shfl_xor_sync(0xffffffffu, sz, o);
+        }
+        if (lane == 0) {
+            origin[0] = 0.5 * sx / (double)t.n_hydros;
+            origin[1] = 0.5 * sz / (double)t.n_hydros;
+        }
     }
-    for (int o = 16; o; o >>= 1) {
-        sx += __shfl_xor_sync(0xffffffffu, sx, o);
-        sz += __shfl_xor_sync(0xffffffffu, sz, o);
-    }
-    const double xx = 0.5 * sx / (double)t.n_hydros, zz = 0.5 * sz / (double)t.n_hydros;
+    __syncthreads();
     const float ku = t.ku, kc = t.kc;
     // |d| is at most a receiver's distance from the origin: whether d/(c dt) of
     // all of them stays below 2^21 samples (the FP32 floor below)
     bool far = false;
     for (int n = threadIdx.x; n < t.n_hydros; n += blockDim.x) {
-        const double x = t.x_r[n], dd = t.D[n];
+        const double x = t.x_r[n], dd = t.D[n], zz = origin[1];
         hyd[n] = make_float2((float)x, (float)(x * x + dd * (dd - 2.0 * zz)));
         far |= !((fabs(x) + fabs(dd) + fabs(zz)) * ku < 2097152.0);
     }
     far = __syncthreads_or(far) || t.n_samples > (1 << 29);
-    const int runs = (t.n_y + 31) / 32;
+    const long long pixels = (long long)t.n_x * t.n_y;
+    const unsigned runs = (unsigned)((pixels + 31) / 32);
+    const int groups = SPLIT ? kTdibWarps / parts : kTdibWarps, group = warp / parts, sub = SPLIT ? warp % parts : 0;
 #pragma unroll 1
-    for (long long wid = (long long)blockIdx.x * kTdibWarps + warp; wid < (long long)t.n_x * runs;
-         wid += (long long)gridDim.x * kTdibWarps) {
-        const int nx = (int)(wid / runs), y0 = (int)(wid % runs) * 32, np = min(32, t.n_y - y0);
-        const int yl = y0 + min(lane, np - 1);   // lanes past the beam's end repeat its last pixel
+    for (unsigned u = blockIdx.x * groups; u < runs; u += gridDim.x * groups) {
+        // a group past the end leaves, or, where its CTA's warps meet, repeats the last
+        // run and stores nothing
+        if (!SPLIT && u + group >= runs) break;
+        const long long g0 = (long long)min(u + group, runs - 1) * 32;
         float a, r, r2, fr, bc;
         int b;
-        {
-            const double X = t.xarr[(size_t)nx * t.n_y + yl], Y = t.yarr[(size_t)nx * t.n_y + yl];
-            const double ax = xx + X, rt2 = ax * ax + Y * Y + zz * zz, rt = sqrt(rt2);
+        if (sub == 0) {
+            const long long gl = min(g0 + lane, pixels - 1);   // lanes past the end repeat the last pixel
+            const double X = t.xarr[gl], Y = t.yarr[gl], zz = origin[1];
+            const double ax = origin[0] + X, rt2 = ax * ax + Y * Y + zz * zz, rt = sqrt(rt2);
             const double tau0 = 2.0 * rt * t.inv_c;
             // a quotient: a delay on the last sample must not come out past it
             const double u0 = (tau0 - t.t0) / t.dt;
@@ -113,6 +136,25 @@ __global__ void __launch_bounds__(32 * kTdibWarps, 4) tdib_kernel(TdibDev t)
             r = (float)rt;
             r2 = (float)rt2;
         }
+        if (SPLIT) {
+            // the group's other warps take them from the first
+            float(*const v)[32] = base[group];
+            if (sub == 0) {
+                v[0][lane] = a;
+                v[1][lane] = r;
+                v[2][lane] = r2;
+                v[3][lane] = fr;
+                v[4][lane] = bc;
+                v[5][lane] = __int_as_float(b);
+            }
+            __syncthreads();
+            a = v[0][lane];
+            r = v[1][lane];
+            r2 = v[2][lane];
+            fr = v[3][lane];
+            bc = v[4][lane];
+            b = __float_as_int(v[5][lane]);
+        }
         const int near = max(min(b, 1 << 30), -(1 << 30));   // no nearer to the axis than b
         const float qnan = __int_as_float(0x7fc00000);
         float2 acc[4];
@@ -120,8 +162,8 @@ __global__ void __launch_bounds__(32 * kTdibWarps, 4) tdib_kernel(TdibDev t)
         for (int q = 0; q < 4; ++q) acc[q] = make_float2(0.f, 0.f);
         auto pass = [&](auto far_c) __attribute__((always_inline)) {
             constexpr bool FAR = decltype(far_c)::value;
-            for (int n0 = 0; n0 < t.n_hydros; n0 += kTdibChunk) {
-                const int nc = min(kTdibChunk, t.n_hydros - n0);
+            for (int n0 = sub * cw; n0 < t.n_hydros; n0 += parts * cw) {
+                const int nc = min(cw, t.n_hydros - n0);
                 // four hydrophones at a time: their gathers in flight together
                 for (int k0 = 0; k0 < nc; k0 += 4) {
                     float2 lo[4], hi[4];
@@ -175,12 +217,13 @@ __global__ void __launch_bounds__(32 * kTdibWarps, 4) tdib_kernel(TdibDev t)
                     }
                 }
                 __syncwarp();
+                const int np = u + group < runs ? (int)min(32LL, pixels - g0) : 0;
                 if (t.Xd) {
                     // two rows of 16 hydrophones a store
-                    const int col = lane % kTdibChunk;
-                    float2 *o = t.Xd + ((size_t)nx * t.n_y + y0) * t.n_hydros + n0 + col;
+                    const int col = lane & (cw - 1);
+                    float2 *o = t.Xd + (size_t)g0 * t.n_hydros + n0 + col;
         #pragma unroll 4
-                    for (int p = lane / kTdibChunk; p < np; p += 32 / kTdibChunk)
+                    for (int p = lane / cw; p < np; p += 32 / cw)
                         if (col < nc) o[(size_t)p * t.n_hydros] = tile[warp][p][col];
                 }
                 __syncwarp();
@@ -188,27 +231,47 @@ __global__ void __launch_bounds__(32 * kTdibWarps, 4) tdib_kernel(TdibDev t)
         };
         if (far) pass(std::true_type{});
         else pass(std::false_type{});
-        if (t.image && lane < np) {
-            const float2 s = cadd(cadd(acc[0], acc[1]), cadd(acc[2], acc[3]));
-            t.image[(size_t)(y0 + lane) * t.n_x + nx] = cscale(s, 1.0f / (float)t.n_hydros);
+        if (t.image) {
+            float2 v = cadd(cadd(acc[0], acc[1]), cadd(acc[2], acc[3]));
+            if (SPLIT) {
+                part[warp][lane] = v;
+                __syncthreads();
+                if (sub == 0)
+                    for (int q = 1; q < parts; ++q) v = cadd(v, part[warp + q][lane]);
+            }
+            if (sub == 0 && u + group < runs && g0 + lane < pixels) {
+                const long long nx = (g0 + lane) / t.n_y, y = g0 + lane - nx * t.n_y;
+                t.image[(size_t)y * t.n_x + nx] = cscale(v, 1.0f / (float)t.n_hydros);
+            }
         }
+        if (SPLIT) __syncthreads();   // the readers of base and part are done
     }
 }
 
 int launch_tdib(const TdibDev &t, cudaStream_t s)
 {
     if (t.n_hydros > kTdibMaxHydros) return cudaErrorNotSupported;
-    const long long warps = (long long)t.n_x * ((t.n_y + 31) / 32);
-    const long long blocks = (warps + kTdibWarps - 1) / kTdibWarps;
-    if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
+    const long long runs = ((long long)t.n_x * t.n_y + 31) / 32;
+    if (runs > 0x7fffffffLL) return cudaErrorInvalidValue;   // 2^36 pixels: 1 TB of coordinates
     int dev = 0, sms = 0, per_sm = 0;
     cudaError_t e;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
         (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess ||
-        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tdib_kernel, 32 * kTdibWarps, 0)) != cudaSuccess)
+        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tdib_kernel<false>, 32 * kTdibWarps, 0)) !=
+            cudaSuccess)
         return e;
     const long long resident = (long long)sms * per_sm;
-    tdib_kernel<<<(unsigned)(blocks < resident ? blocks : resident), 32 * kTdibWarps, 0, s>>>(t);
+    // few pixels: a warp's time is that of its hydrophones, one batch of four after
+    // the other, so as many warps as would be idle share them
+    int parts = 1;
+    while (parts < kTdibWarps && runs * parts * 2 <= resident * kTdibWarps && parts * 4 < t.n_hydros) parts *= 2;
+    const int each = (t.n_hydros + parts - 1) / parts, cw = each <= 4 ? 4 : each <= 8 ? 8 : kTdibChunk;
+    const long long groups = kTdibWarps / parts, blocks = (runs + groups - 1) / groups;
+    const unsigned grid = (unsigned)(blocks < resident ? blocks : resident);
+    if (parts > 1)
+        tdib_kernel<true><<<grid, 32 * kTdibWarps, 0, s>>>(t, parts, cw);
+    else
+        tdib_kernel<false><<<grid, 32 * kTdibWarps, 0, s>>>(t, 1, kTdibChunk);
     return cudaGetLastError();
 }
 
