@@ -176,150 +176,159 @@ COS_DEV void async_copy8(void *dst, const void *src, bool is)
                  : "memory");
 }
 
-// window rows t0 .. t0+T-1 (T <= 32, a lane each); a longer window, or one whose
-// accumulators leave fewer than two CTAs an SM, takes several launches (backward pass
-// at M=128, L=32, K=4, [64][520]: 840 -> 640 us; M=33, L=16, K=17: 444 -> 354 us, both against
-// register-blocked tiles)
+// `per` window rows at a time (at most 32, a lane each): a longer window, or one whose
+// accumulators leave fewer than two CTAs an SM, takes several passes over the rows, whose
+// gradients add up (backward pass at M=128, L=32, K=4, [64][520]: 840 -> 640 us; M=33, L=16,
+// K=17: 444 -> 354 us, both against register-blocked tiles).  A row none of whose pixels
+// has a gradient is not staged: the gradients are read two rows ahead.
 template <int L, int SB>
-__global__ void __launch_bounds__(32 * kRowWarps, 2) adjoint_row_kernel(AdjDev a, int t0, int T)
+__global__ void __launch_bounds__(32 * kRowWarps, 2) adjoint_row_kernel(AdjDev a, int per)
 {
     static_assert(SB % 2 == 0 && L % 2 == 0, "channel pairs are 16 bytes");
     extern __shared__ __align__(16) unsigned char smraw[];
     const int M = a.M, Ns = M - L + 1;
-    const AdjRowSmem S(M, L, T, SB);
+    const AdjRowSmem S(M, L, per, SB);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned char *const mine = smraw + warp * S.per_warp;
     float2 *const acc = (float2 *)(mine + S.off_a);
     float *const ths = (float *)(smraw + kRowWarps * S.per_warp) + (size_t)warp * M;   // channel-phase sums
     const float scale = 1.0f / ((float)Ns * (float)(2 * a.K + 1));
-    const int nsb = (Ns + SB - 1) / SB, items = T * nsb;
+    const int nsb = (Ns + SB - 1) / SB;
     float dacc = 0.f;
     for (int c = lane; c < M; c += 32) ths[c] = 0.f;
     for (int b = 0; b < 2; ++b) {   // the zero tails: samples past M, weights of the lanes without an item
         for (int c = M + lane; c < S.xs; c += 32) ((float2 *)mine)[b * S.xs + c] = make_float2(0.f, 0.f);
         for (int l = lane; l < L; l += 32)
-            ((float2 *)(mine + S.off_w))[(b * (T + 1) + T) * S.ws + l] = make_float2(0.f, 0.f);
+            ((float2 *)(mine + S.off_w))[(b * (per + 1) + per) * S.ws + l] = make_float2(0.f, 0.f);
     }
     const long long rows = (long long)a.Nx * a.Ny, step = (long long)gridDim.x * kRowWarps;
-    // gradient of pixel y-t0-t on lane t; 0 where there is none
-    auto grad = [&](long long row) {
-        const int bx = (int)(row / a.Ny), p = (int)(row % a.Ny) - t0 - lane;
-        return row < rows && lane < T && p >= 0 && p < a.Npy ? a.gP[(size_t)bx * a.Npy + p] : 0.f;
-    };
-    // the row's samples and the weights of its pixels (zeros where there is none)
-    // into buffer b
-    auto stage = [&](long long row, int b) {
-        const int bx = (int)(row / a.Ny), y = (int)(row % a.Ny);
-        float2 *const xd = (float2 *)mine + b * S.xs, *const wd = (float2 *)(mine + S.off_w) + b * (T + 1) * S.ws;
-        const float2 *xr = a.x + (size_t)row * M;
-        for (int c = lane; c < M; c += 32) async_copy8(xd + c, xr + c, true);
-        for (int i = lane; i < T * L; i += 32) {
-            const int t = i / L, l = i % L, p = y - t0 - t;
-            const bool is = p >= 0 && p < a.Npy;
-            async_copy8(wd + t * S.ws + l, a.w + ((size_t)bx * a.Npy + (is ? p : 0)) * L + l, is);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    long long row = (long long)blockIdx.x * kRowWarps + warp;
-    float gnext = grad(row);
-    if (row < rows) stage(row, 0);
-    int b = 0;
-    for (; row < rows; row += step, b ^= 1) {
-        const float gl = gnext;
-        gnext = grad(row + step);
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncwarp();   // the row has arrived for every lane, and the last one's readers are done
-        if (row + step < rows) stage(row + step, b ^ 1);
-        const float2 *const xw = (const float2 *)mine + b * S.xs;
-        float2 *const ws = (float2 *)(mine + S.off_w) + b * (T + 1) * S.ws;
-        // a pixel without a gradient takes no part, its weights finite or not; a row
-        // of such pixels gets nothing
-        const unsigned on = __ballot_sync(0xffffffffu, gl != 0.f);
-        if (on == 0u) continue;
-        for (int t = 0; t < T; ++t)
-            if (!(on >> t & 1u))
-                for (int l = lane; l < L; l += 32) ws[t * S.ws + l] = make_float2(0.f, 0.f);
-        for (int i = lane; i < (T + 1) * S.as; i += 32) acc[i] = make_float2(0.f, 0.f);
-        __syncwarp();
-        for (int it0 = 0; it0 < items; it0 += 32) {
-            const int it = it0 + lane, t = it < items ? it / nsb : T, s0 = it < items ? (it - t * nsb) * SB : 0;
-            const float gt = __shfl_sync(0xffffffffu, gl, t < T ? t : 0), g = t < T ? gt : 0.f;
-            float2 w[L];
-#pragma unroll
-            for (int l = 0; l < L; l += 2) {
-                const float4 v = *(const float4 *)(ws + t * S.ws + l);
-                w[l] = make_float2(v.x, v.y);
-                w[l + 1] = make_float2(v.z, v.w);
+#pragma unroll 1
+    for (int t0 = 0; t0 < 2 * a.K + 1; t0 += per) {
+        const int T = min(per, 2 * a.K + 1 - t0), items = T * nsb;   // window rows t0 .. t0+T-1
+        // gradient of pixel y-t0-t on lane t; 0 where there is none
+        auto grad = [&](long long row) {
+            const int bx = (int)(row / a.Ny), p = (int)(row % a.Ny) - t0 - lane;
+            return row < rows && lane < T && p >= 0 && p < a.Npy ? a.gP[(size_t)bx * a.Npy + p] : 0.f;
+        };
+        // the row's samples and the weights of its pixels (zeros where there is none)
+        // into buffer b
+        auto stage = [&](long long row, int b) {
+            const int bx = (int)(row / a.Ny), y = (int)(row % a.Ny);
+            float2 *const xd = (float2 *)mine + b * S.xs, *const wd = (float2 *)(mine + S.off_w) + b * (per + 1) * S.ws;
+            const float2 *xr = a.x + (size_t)row * M;
+            for (int c = lane; c < M; c += 32) async_copy8(xd + c, xr + c, true);
+            for (int i = lane; i < T * L; i += 32) {
+                const int t = i / L, l = i % L, p = y - t0 - t;
+                const bool is = p >= 0 && p < a.Npy;
+                async_copy8(wd + t * S.ws + l, a.w + ((size_t)bx * a.Npy + (is ? p : 0)) * L + l, is);
             }
-            if (t0 == 0 && it < nsb) {   // pixel y; one lane adds g |w|^2
-                float wn = 0.f;
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        long long row = (long long)blockIdx.x * kRowWarps + warp;
+        float gnext = grad(row), gafter = grad(row + step);
+        unsigned next = __ballot_sync(0xffffffffu, gnext != 0.f);
+        __syncwarp();   // the last pass' readers are done
+        if (next) stage(row, 0);
+        int b = 0;
+        for (; row < rows; row += step, b ^= 1) {
+            const float gl = gnext;
+            gnext = gafter;
+            gafter = grad(row + 2 * step);
+            // a pixel without a gradient takes no part, its weights finite or not; a row
+            // of such pixels gets nothing
+            const unsigned on = next;
+            next = __ballot_sync(0xffffffffu, gnext != 0.f);
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncwarp();   // the row has arrived for every lane, and the last one's readers are done
+            if (next) stage(row + step, b ^ 1);
+            if (on == 0u) continue;
+            const float2 *const xw = (const float2 *)mine + b * S.xs;
+            float2 *const ws = (float2 *)(mine + S.off_w) + b * (per + 1) * S.ws;
+            for (int t = 0; t < T; ++t)
+                if (!(on >> t & 1u))
+                    for (int l = lane; l < L; l += 32) ws[t * S.ws + l] = make_float2(0.f, 0.f);
+            for (int i = lane; i < (T + 1) * S.as; i += 32) acc[i] = make_float2(0.f, 0.f);
+            __syncwarp();
+            for (int it0 = 0; it0 < items; it0 += 32) {
+                const int it = it0 + lane, t = it < items ? it / nsb : per, s0 = it < items ? (it - t * nsb) * SB : 0;
+                const float gt = __shfl_sync(0xffffffffu, gl, t < T ? t : 0), g = t < T ? gt : 0.f;
+                float2 w[L];
 #pragma unroll
-                for (int l = 0; l < L; ++l) wn += cabs2(w[l]);
-                if (it == 0) dacc += g * wn;
-            }
-            // e_s, s = s0 .. s0+SB-1: (re, im) parts as pair sums
-            float2 er[SB], ei[SB];
+                for (int l = 0; l < L; l += 2) {
+                    const float4 v = *(const float4 *)(ws + t * S.ws + l);
+                    w[l] = make_float2(v.x, v.y);
+                    w[l + 1] = make_float2(v.z, v.w);
+                }
+                if (t0 == 0 && it < nsb) {   // pixel y; one lane adds g |w|^2
+                    float wn = 0.f;
 #pragma unroll
-            for (int j = 0; j < SB; ++j) er[j] = ei[j] = make_float2(0.f, 0.f);
+                    for (int l = 0; l < L; ++l) wn += cabs2(w[l]);
+                    if (it == 0) dacc += g * wn;
+                }
+                // e_s, s = s0 .. s0+SB-1: (re, im) parts as pair sums
+                float2 er[SB], ei[SB];
 #pragma unroll
-            for (int i = 0; i < SB + L - 1; i += 2) {
-                const float4 q = *(const float4 *)(xw + s0 + i);
+                for (int j = 0; j < SB; ++j) er[j] = ei[j] = make_float2(0.f, 0.f);
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const float2 v = h ? make_float2(q.z, q.w) : make_float2(q.x, q.y);
-                    const float2 u = make_float2(v.y, -v.x);
+                for (int i = 0; i < SB + L - 1; i += 2) {
+                    const float4 q = *(const float4 *)(xw + s0 + i);
 #pragma unroll
-                    for (int j = 0; j < SB; ++j) {
-                        const int l = i + h - j;
-                        if (l >= 0 && l < L) {
-                            // conj(w) v = (w.re v.re + w.im v.im, w.re v.im - w.im v.re)
-                            er[j] = ffma2(w[l], v, er[j]);
-                            ei[j] = ffma2(w[l], u, ei[j]);
+                    for (int h = 0; h < 2; ++h) {
+                        const float2 v = h ? make_float2(q.z, q.w) : make_float2(q.x, q.y);
+                        const float2 u = make_float2(v.y, -v.x);
+#pragma unroll
+                        for (int j = 0; j < SB; ++j) {
+                            const int l = i + h - j;
+                            if (l >= 0 && l < L) {
+                                // conj(w) v = (w.re v.re + w.im v.im, w.re v.im - w.im v.re)
+                                er[j] = ffma2(w[l], v, er[j]);
+                                ei[j] = ffma2(w[l], u, ei[j]);
+                            }
                         }
                     }
                 }
-            }
-            // e_s g / (Ns T) as (re, -im) and (im, re)
-            const float gs = g * scale;
+                // e_s g / (Ns T) as (re, -im) and (im, re)
+                const float gs = g * scale;
 #pragma unroll
-            for (int j = 0; j < SB; ++j) {
-                const bool in = s0 + j < Ns;
-                const float re = in ? (er[j].x + er[j].y) * gs : 0.f, im = in ? (ei[j].x + ei[j].y) * gs : 0.f;
-                er[j] = make_float2(re, -im);
-                ei[j] = make_float2(im, re);
-            }
-            float2 *const at = acc + t * S.as + s0;
-#pragma unroll
-            for (int i = 0; i < SB + L - 1; i += 2) {
-                float2 G[2];
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    float2 pr = make_float2(0.f, 0.f), pi = pr;
-#pragma unroll
-                    for (int j = 0; j < SB; ++j) {
-                        const int l = i + h - j;
-                        if (l >= 0 && l < L) {
-                            pr = ffma2(er[j], w[l], pr);
-                            pi = ffma2(ei[j], w[l], pi);
-                        }
-                    }
-                    G[h] = make_float2(pr.x + pr.y, pi.x + pi.y);
+                for (int j = 0; j < SB; ++j) {
+                    const bool in = s0 + j < Ns;
+                    const float re = in ? (er[j].x + er[j].y) * gs : 0.f, im = in ? (ei[j].x + ei[j].y) * gs : 0.f;
+                    er[j] = make_float2(re, -im);
+                    ei[j] = make_float2(im, re);
                 }
-                float4 *const d = (float4 *)(at + i);
-                const float4 o = *d;
-                *d = make_float4(o.x + G[0].x, o.y + G[0].y, o.z + G[1].x, o.w + G[1].y);
-                __syncwarp();
+                float2 *const at = acc + min(t, T) * S.as + s0;   // lanes without an item: past the last
+#pragma unroll
+                for (int i = 0; i < SB + L - 1; i += 2) {
+                    float2 G[2];
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        float2 pr = make_float2(0.f, 0.f), pi = pr;
+#pragma unroll
+                        for (int j = 0; j < SB; ++j) {
+                            const int l = i + h - j;
+                            if (l >= 0 && l < L) {
+                                pr = ffma2(er[j], w[l], pr);
+                                pi = ffma2(ei[j], w[l], pi);
+                            }
+                        }
+                        G[h] = make_float2(pr.x + pr.y, pi.x + pi.y);
+                    }
+                    float4 *const d = (float4 *)(at + i);
+                    const float4 o = *d;
+                    *d = make_float4(o.x + G[0].x, o.y + G[0].y, o.z + G[1].x, o.w + G[1].y);
+                    __syncwarp();
+                }
             }
-        }
-        // the row's gradient, and its share of the channel phases
-        float2 *gout = a.gx + (size_t)row * M;
-        for (int c = lane; c < M; c += 32) {
-            float2 G = acc[c];
-            for (int t = 1; t < T; ++t) G = cadd(G, acc[t * S.as + c]);
-            const float2 xv = xw[c];
-            ths[c] += 2.f * (G.x * xv.y - G.y * xv.x);
-            // added without waiting for the old value
-            asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(gout + c), "f"(G.x), "f"(G.y) : "memory");
+            // the row's gradient, and its share of the channel phases
+            float2 *gout = a.gx + (size_t)row * M;
+            for (int c = lane; c < M; c += 32) {
+                float2 G = acc[c];
+                for (int t = 1; t < T; ++t) G = cadd(G, acc[t * S.as + c]);
+                const float2 xv = xw[c];
+                ths[c] += 2.f * (G.x * xv.y - G.y * xv.x);
+                // added without waiting for the old value
+                asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(gout + c), "f"(G.x), "f"(G.y) : "memory");
+            }
         }
     }
     if (a.gd && lane == 0 && dacc != 0.f) atomicAdd(a.gd, dacc);
@@ -349,17 +358,16 @@ static int launch_adjoint_with(Kern kern, const AdjDev &a, long long units, size
     return cudaGetLastError();
 }
 
-// window rows a launch of the row kernel takes: at most 32 (a lane each) and what
-// leaves two CTAs an SM, spread evenly over the launches; the gradient rows add up.
-// 0: not even one row fits so
-static int rows_per_launch(const AdjDev &a)
+// window rows a pass of the row kernel takes: at most 32 (a lane each) and what
+// leaves two CTAs an SM, spread evenly over the passes.  0: not even one row fits so
+static int rows_per_pass(const AdjDev &a)
 {
     const int T = 2 * a.K + 1;
     int most = T < 32 ? T : 32;
     while (most > 0 && AdjRowSmem(a.M, a.L, most, 8).total > 112 * 1024) --most;
     if (most == 0) return 0;
-    const int launches = (T + most - 1) / most;
-    return (T + launches - 1) / launches;
+    const int passes = (T + most - 1) / most;
+    return (T + passes - 1) / passes;
 }
 
 // SB: the block length that keeps the lanes fullest, passes of 32 items by the
@@ -368,23 +376,18 @@ template <int L>
 static int launch_rows(const AdjDev &a, int per, int num_sms, cudaStream_t s)
 {
     static_assert(kRowWarps == kAdjWarps, "one launch helper");
-    const int T = 2 * a.K + 1, Ns = a.M - L + 1;
+    const int Ns = a.M - L + 1;
     const long long units = ((long long)a.Nx * a.Ny + kRowWarps - 1) / kRowWarps;
     auto cost = [&](int sb) { return (per * ((Ns + sb - 1) / sb) + 31) / 32 * (sb + 2); };
     int best = 2;
     for (int sb : {4, 6, 8})
         if (cost(sb) < cost(best)) best = sb;
-    for (int t0 = 0; t0 < T; t0 += per) {
-        const int n = T - t0 < per ? T - t0 : per;
-        const size_t smem = AdjRowSmem(a.M, L, n, best).total;
-        auto go = [&](auto kern) { return launch_adjoint_with(kern, a, units, smem, num_sms, s, t0, n); };
-        const int e = best == 2   ? go(adjoint_row_kernel<L, 2>)
-                      : best == 4 ? go(adjoint_row_kernel<L, 4>)
-                      : best == 6 ? go(adjoint_row_kernel<L, 6>)
-                                  : go(adjoint_row_kernel<L, 8>);
-        if (e) return e;
-    }
-    return 0;
+    const size_t smem = AdjRowSmem(a.M, L, per, best).total;
+    auto go = [&](auto kern) { return launch_adjoint_with(kern, a, units, smem, num_sms, s, per); };
+    return best == 2   ? go(adjoint_row_kernel<L, 2>)
+           : best == 4 ? go(adjoint_row_kernel<L, 4>)
+           : best == 6 ? go(adjoint_row_kernel<L, 6>)
+                       : go(adjoint_row_kernel<L, 8>);
 }
 
 int launch_adjoint(const AdjDev &a, int num_sms, cudaStream_t s)
@@ -394,7 +397,7 @@ int launch_adjoint(const AdjDev &a, int num_sms, cudaStream_t s)
                         (size_t)kAdjWarps * (a.L + T * Ns) * sizeof(float2);
     if (smem > 227 * 1024 || a.L > 64) return cudaErrorNotSupported;
     // by rows; the tiles serve the other subarray lengths
-    if (const int per = rows_per_launch(a)) {
+    if (const int per = rows_per_pass(a)) {
         switch (a.L) {
         case 8: return launch_rows<8>(a, per, num_sms, s);
         case 16: return launch_rows<16>(a, per, num_sms, s);
