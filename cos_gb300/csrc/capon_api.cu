@@ -61,8 +61,21 @@ struct cos_capon_ctx {
     DevBuf A, b, sol;
     DevBuf V;           // subspace matrix of the host-pointer subspace call
     DevBuf tdib_in;     // inputs of the host-pointer steering call
-    // autotuner: chosen fused candidate per (L, K, M, FusedMode)
-    std::map<std::tuple<int, int, int, int>, int> tuned;
+    // autotuner: chosen fused candidate per (L, K, M, FusedMode), and the pixels of
+    // the launch that it was timed on
+    struct Choice {
+        int cand;
+        long long pixels;
+    };
+    std::map<std::tuple<int, int, int, int>, Choice> tuned;
+    // whether the choice for a shape holds for a launch of that many pixels: made on
+    // at least a quarter as many, or on enough of them that the times tell the
+    // candidates apart (a few tiles an SM; 62 pixels take every candidate about 10 us)
+    bool tuned_for(const std::tuple<int, int, int, int> &key, long long pixels) const
+    {
+        const auto it = tuned.find(key);
+        return it != tuned.end() && (it->second.pixels >= 65536 || pixels <= 4 * it->second.pixels);
+    }
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // second stream of the pipelined host-pointer call
     cudaStream_t stream2 = nullptr;
@@ -180,9 +193,10 @@ static bool use_fused(const FrameDev &f, const cos_capon_opts &o)
 // Autotuner: the first launch of an (L, K, M, mode) shape on a context times
 // every candidate configuration on the frames themselves (each candidate
 // computes the same per-pixel arithmetic), keeps the fastest, and reruns it so
-// that the outputs are the winner's.  COS_CAPON_FUSED_CONFIG=<name> forces a
-// candidate.  While the stream is being captured into a graph no timing is
-// possible, so an untuned shape then takes the first candidate.
+// that the outputs are the winner's; a choice made on few pixels is made again for
+// a much larger launch (cos_capon_ctx::tuned_for).  COS_CAPON_FUSED_CONFIG=<name>
+// forces a candidate.  While the stream is being captured into a graph no timing is
+// possible: the choice there is, or for an untuned shape the first candidate.
 static int launch_fused_tuned(cos_capon_ctx *c, const FramesParam &fp, int mode, int form, cudaStream_t s)
 {
     const FrameDev &f0 = fp.f[0];
@@ -200,11 +214,13 @@ static int launch_fused_tuned(cos_capon_ctx *c, const FramesParam &fp, int mode,
             if (!strcmp(force, cand[i].name)) return cand[i].launch(fp, mode, c->d_status, c->num_sms, s);
     }
     const auto key = std::make_tuple(f0.L, f0.K, f0.M, mode | (form << 8));
+    long long pixels = 0;
+    for (int q = 0; q < fp.n; ++q) pixels += (long long)fp.f[q].Nx * fp.f[q].Npy;
     auto it = c->tuned.find(key);
-    if (it != c->tuned.end()) return cand[it->second].launch(fp, mode, c->d_status, c->num_sms, s);
+    if (c->tuned_for(key, pixels)) return cand[it->second.cand].launch(fp, mode, c->d_status, c->num_sms, s);
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone || ok.size() == 1)
-        return cand[ok[0]].launch(fp, mode, c->d_status, c->num_sms, s);
+        return cand[it != c->tuned.end() ? it->second.cand : ok[0]].launch(fp, mode, c->d_status, c->num_sms, s);
     if (!c->ev0) {
         if (cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess) {
             cudaGetLastError();
@@ -237,7 +253,7 @@ static int launch_fused_tuned(cos_capon_ctx *c, const FramesParam &fp, int mode,
             best = i;
         }
     }
-    c->tuned[key] = best;
+    c->tuned[key] = {best, pixels};
     if (getenv("COS_CAPON_TUNE_VERBOSE")) fprintf(stderr, "[cos_capon] L=%d K=%d M=%d mode=%d -> %s (%.3f ms)\n",
                                                   f0.L, f0.K, f0.M, mode, cand[best].name, best_ms);
     return cand[best].launch(fp, mode, c->d_status, c->num_sms, s);
@@ -444,8 +460,10 @@ static int run_frames(cos_capon_ctx *c, const FrameDev *fs, int n, const cos_cap
         if (g.kind == 0) {
             const FrameDev &f = fs[g.first];
             const int mode = g.mode();
-            tuned_all &= c->tuned.count(std::make_tuple(f.L, f.K, f.M, mode | (o.form << 8))) != 0;
-            if (g.want_R) tuned_all &= c->tuned.count(std::make_tuple(f.L, f.K, f.M, FUSED_R | (o.form << 8))) != 0;
+            long long pixels = 0;
+            for (int q = 0; q < g.count; ++q) pixels += (long long)fs[g.first + q].Nx * fs[g.first + q].Npy;
+            tuned_all &= c->tuned_for(std::make_tuple(f.L, f.K, f.M, mode | (o.form << 8)), pixels);
+            if (g.want_R) tuned_all &= c->tuned_for(std::make_tuple(f.L, f.K, f.M, FUSED_R | (o.form << 8)), pixels);
         }
     }
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -647,7 +665,8 @@ static int get_capon_host(cos_capon_ctx *c, void *z, float *P, void *w, void *R,
     // runs whole, so the autotuner times the frame once, on one stream.
     const bool fused = use_fused(make_frame(probe, o), o);
     const bool no_scratch = (fused && !o.refine) || Nb > 0 || sliding;
-    const bool tuned = !fused || c->tuned.count(std::make_tuple(L, Yavg, M, (int)(w ? FUSED_W : FUSED_ZP) | (o.form << 8)));
+    const bool tuned = !fused || c->tuned_for(std::make_tuple(L, Yavg, M, (int)(w ? FUSED_W : FUSED_ZP) | (o.form << 8)),
+                                              (long long)npix);
     if (no_scratch && tuned && !R && !V && Nx >= 4 && is_pinned(x) && is_pinned(z) && (!P || is_pinned(P)) &&
         (!w || is_pinned(w))) {
         if (!c->stream2 && cudaStreamCreateWithFlags(&c->stream2, cudaStreamNonBlocking) != cudaSuccess) {
