@@ -293,7 +293,7 @@ COS_DEV float2 bs_ff_residual(float2 a, float2 h, float2 l)
 //            the half-warp in float-float -> Q_row (Nb x Nb upper, hi + lo),
 //            the row's snapshot energy and beam sums sum_s Y_s;
 //   phase B  one thread per pixel: R_bs = sum of the window's Q rows
-//            (float-float), loading, FP32 Cholesky, one FP64-residual
+//            (float-float), loading, FP32 Cholesky, one float-float-residual
 //            refinement step, P and z (g_bs = B g = the centre row's beam sums / Ns);
 //   phase C  (w requested) w = B^H x_bs / a_bs^H x_bs, one thread per output.
 static constexpr int kTileThreads = 256;
@@ -732,9 +732,6 @@ struct BsWideSmem {
     }
 };
 
-// i / d by the reciprocal of d; exact while the quotient times d stays below 2^21
-COS_DEV int bs_div(int i, float inv) { return (int)(((float)i + 0.5f) * inv); }
-
 template <int G>
 __global__ void __launch_bounds__(kWideThreads, 2)
 beamspace_wide_kernel(FrameDev f, float2 *__restrict__ Rbs, int tile, int units)
@@ -799,7 +796,7 @@ beamspace_wide_kernel(FrameDev f, float2 *__restrict__ Rbs, int tile, int units)
             const int nch = (Ns + 2) / 3, nbp = NbE / 2;
             const float inv_nbp = 1.f / (float)nbp, inv_nch = 1.f / (float)nch;
             for (int it = tid; it < rows * nch * nbp; it += kWideThreads) {
-                const int rc = bs_div(it, inv_nbp), b = 2 * (it - rc * nbp), r = bs_div(rc, inv_nch), ch = rc - r * nch;
+                const int rc = small_div(it, inv_nbp), b = 2 * (it - rc * nbp), r = small_div(rc, inv_nch), ch = rc - r * nch;
                 // direct in the chunk's middle, one step of the recurrence either way
                 const int s0 = ch * 3, sc = min(s0 + 1, Ns - 1);
                 const float2 *xr = xs + (size_t)r * M + sc;
@@ -850,7 +847,7 @@ beamspace_wide_kernel(FrameDev f, float2 *__restrict__ Rbs, int tile, int units)
         {
             const float inv_nt = 1.f / (float)nt, inv_nb = 1.f / (float)Nb;
             for (int it = tid; it < rows * nt; it += kWideThreads) {
-                const int r = bs_div(it, inv_nt), e = blk[it - r * nt];
+                const int r = small_div(it, inv_nt), e = blk[it - r * nt];
                 const int bi = e >> 8, bj = e & 255;
                 const float2 *y = Y + (size_t)r * Ns * NbE;
                 float2 hi[4], lo[4];
@@ -890,7 +887,7 @@ beamspace_wide_kernel(FrameDev f, float2 *__restrict__ Rbs, int tile, int units)
             }
             // beam sums of the row
             for (int it = tid; it < rows * Nb; it += kWideThreads) {
-                const int r = bs_div(it, inv_nb), b = it - r * Nb;
+                const int r = small_div(it, inv_nb), b = it - r * Nb;
                 float2 g0 = make_float2(0.f, 0.f), g1 = g0;
                 const float2 *y = Y + (size_t)r * Ns * NbE + b;
                 int s = 0;
@@ -907,7 +904,7 @@ beamspace_wide_kernel(FrameDev f, float2 *__restrict__ Rbs, int tile, int units)
         // ---- window sums, renormalised: (value, remainder)
         const float inv_nq = 1.f / (float)NQ;
         for (int it = tid; it < np * NQ; it += kWideThreads) {
-            const int lp = bs_div(it, inv_nq), e = it - lp * NQ;
+            const int lp = small_div(it, inv_nq), e = it - lp * NQ;
             float2 h = make_float2(0.f, 0.f), l = h;
             for (int t = 0; t < T; ++t) {
                 const float4 q = Qs[(size_t)(lp + t) * NQ + e];
@@ -1044,7 +1041,7 @@ beamspace_wide_kernel(FrameDev f, float2 *__restrict__ Rbs, int tile, int units)
             // w = B^H x_bs / sum, one thread per (pixel, element)
             const float inv_l = 1.f / (float)L;
             for (int i = tid; i < np * L; i += kWideThreads) {
-                const int lp = bs_div(i, inv_l), l = i - lp * L;
+                const int lp = small_div(i, inv_l), l = i - lp * L;
                 const float2 *xv = Xb + (size_t)lp * (Nb + 1), *bl = Bt + l * NbE;
                 float2 ria = make_float2(0.f, 0.f);
                 for (int b = 0; b < Nb; ++b) ria = cmac4_conj(ria, bl[b], xv[b]);

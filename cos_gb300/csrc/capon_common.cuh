@@ -96,6 +96,9 @@ COS_DEV void two_sum_acc(float2 &hi, float2 &lo, float2 v)
     lo = fadd2(lo, e);
 }
 
+// i / d by the reciprocal of d; exact while the quotient times d stays below 2^21
+COS_DEV int small_div(int i, float inv) { return (int)(((float)i + 0.5f) * inv); }
+
 // ---- warp helpers ---------------------------------------------------------
 COS_DEV float2 shfl2(float2 v, int src, int width)
 {

@@ -213,8 +213,7 @@ fused_kernel(const __grid_constant__ FramesParam fp, long long total_units, unsi
         const float invM = 1.0f / (float)M;
         for (int i = tid; i < rows * M; i += nthreads) {
             const float2 v = direct ? src[i] : raw[b][i];
-            // i / M: by the reciprocal (exact below 2^21) where M is not a constant
-            const int rr = C::M ? i / M : (int)(((float)i + 0.5f) * invM), cc = C::M ? i % M : i - rr * M;
+            const int rr = C::M ? i / M : small_div(i, invM), cc = C::M ? i % M : i - rr * M;
             xe[rr * XS + cc] = make_float4(v.x, v.y, v.y, -v.x);
         }
         __syncthreads();

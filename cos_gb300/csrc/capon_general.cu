@@ -82,9 +82,6 @@ struct CovShape {
     }
 };
 
-// i / d by the reciprocal of d; exact while the quotient times d stays below 2^21
-COS_DEV int small_div(int i, float inv) { return (int)(((float)i + 0.5f) * inv); }
-
 // (h, l) += a b, componentwise, the product exact: TwoSum with the rounded product,
 // whose own error comes with its last difference, a b - bb, in one fma
 COS_DEV void ff_fma2(float2 &h, float2 &l, float2 a, float2 b)

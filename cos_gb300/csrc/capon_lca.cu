@@ -57,8 +57,7 @@ __global__ void __launch_bounds__(kLcaThreads, 3) lca_kernel(LcaDev a)
 #pragma unroll 5
         for (int i = tid; i < rows * cols * (4 * Q); i += kLcaThreads) {
             const int px = i / (4 * Q), w = i % (4 * Q);
-            // px / cols by the reciprocal: exact below 2^21
-            const int r = (int)(((float)px + 0.5f) * inv);
+            const int r = small_div(px, inv);
             const int yy = y0 - a.Ymid + r, xx = x0 - a.Xmid + px - r * cols;
             float v = 0.f;
             if (w < nw && yy >= 0 && yy < a.Ny && xx >= 0 && xx < a.Nx)
