@@ -194,26 +194,31 @@ __global__ void __launch_bounds__(32 * kRowWarps, 2) adjoint_row_kernel(AdjDev a
     float *const ths = (float *)(smraw + kRowWarps * S.per_warp) + (size_t)warp * M;   // channel-phase sums
     const float scale = 1.0f / ((float)Ns * (float)(2 * a.K + 1));
     const int nsb = (Ns + SB - 1) / SB;
-    float dacc = 0.f;
+    // a warp's sum of g |w|^2.  Its terms cancel (gradients of either sign), so they are
+    // added in FP64, one a row, and a CTA's sum goes out once
+    __shared__ double dsum[kRowWarps];
+    if (lane == 0) dsum[warp] = 0.0;
     for (int c = lane; c < M; c += 32) ths[c] = 0.f;
     for (int b = 0; b < 2; ++b) {   // the zero tails: samples past M, weights of the lanes without an item
         for (int c = M + lane; c < S.xs; c += 32) ((float2 *)mine)[b * S.xs + c] = make_float2(0.f, 0.f);
         for (int l = lane; l < L; l += 32)
             ((float2 *)(mine + S.off_w))[(b * (per + 1) + per) * S.ws + l] = make_float2(0.f, 0.f);
     }
-    const long long rows = (long long)a.Nx * a.Ny, step = (long long)gridDim.x * kRowWarps;
+    const unsigned rows = (unsigned)a.Nx * a.Ny, step = gridDim.x * kRowWarps;
 #pragma unroll 1
     for (int t0 = 0; t0 < 2 * a.K + 1; t0 += per) {
         const int T = min(per, 2 * a.K + 1 - t0), items = T * nsb;   // window rows t0 .. t0+T-1
         // gradient of pixel y-t0-t on lane t; 0 where there is none
-        auto grad = [&](long long row) {
-            const int bx = (int)(row / a.Ny), p = (int)(row % a.Ny) - t0 - lane;
+        auto grad = [&](unsigned row) {
+            const unsigned bx = row / (unsigned)a.Ny;
+            const int p = (int)(row - bx * a.Ny) - t0 - lane;
             return row < rows && lane < T && p >= 0 && p < a.Npy ? a.gP[(size_t)bx * a.Npy + p] : 0.f;
         };
         // the row's samples and the weights of its pixels (zeros where there is none)
         // into buffer b
-        auto stage = [&](long long row, int b) {
-            const int bx = (int)(row / a.Ny), y = (int)(row % a.Ny);
+        auto stage = [&](unsigned row, int b) {
+            const unsigned bx = row / (unsigned)a.Ny;
+            const int y = (int)(row - bx * a.Ny);
             float2 *const xd = (float2 *)mine + b * S.xs, *const wd = (float2 *)(mine + S.off_w) + b * (per + 1) * S.ws;
             const float2 *xr = a.x + (size_t)row * M;
             for (int c = lane; c < M; c += 32) async_copy8(xd + c, xr + c, true);
@@ -224,7 +229,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 2) adjoint_row_kernel(AdjDev a
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
-        long long row = (long long)blockIdx.x * kRowWarps + warp;
+        unsigned row = blockIdx.x * kRowWarps + warp;
         float gnext = grad(row), gafter = grad(row + step);
         unsigned next = __ballot_sync(0xffffffffu, gnext != 0.f);
         __syncwarp();   // the last pass' readers are done
@@ -263,7 +268,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 2) adjoint_row_kernel(AdjDev a
                     float wn = 0.f;
 #pragma unroll
                     for (int l = 0; l < L; ++l) wn += cabs2(w[l]);
-                    if (it == 0) dacc += g * wn;
+                    if (it == 0) dsum[warp] += (double)(g * wn);   // lane 0's
                 }
                 // e_s, s = s0 .. s0+SB-1: (re, im) parts as pair sums
                 float2 er[SB], ei[SB];
@@ -331,8 +336,12 @@ __global__ void __launch_bounds__(32 * kRowWarps, 2) adjoint_row_kernel(AdjDev a
             }
         }
     }
-    if (a.gd && lane == 0 && dacc != 0.f) atomicAdd(a.gd, dacc);
     __syncthreads();
+    if (a.gd && threadIdx.x == 0) {
+        double v = 0.0;
+        for (int k = 0; k < kRowWarps; ++k) v += dsum[k];
+        if (v != 0.0) atomicAdd(a.gd, (float)v);
+    }
     if (a.gth) {
         const float *all = (const float *)(smraw + kRowWarps * S.per_warp);
         for (int c = threadIdx.x; c < M; c += blockDim.x) {
@@ -396,8 +405,10 @@ int launch_adjoint(const AdjDev &a, int num_sms, cudaStream_t s)
     const size_t smem = (size_t)2 * rows * a.M * sizeof(float2) + (size_t)((a.M + 1) & ~1) * sizeof(float) +
                         (size_t)kAdjWarps * (a.L + T * Ns) * sizeof(float2);
     if (smem > 227 * 1024 || a.L > 64) return cudaErrorNotSupported;
-    // by rows; the tiles serve the other subarray lengths
-    if (const int per = rows_per_pass(a)) {
+    // by rows (counted in 32 bits, two steps of the grid ahead); the tiles serve the other
+    // subarray lengths
+    const int per = (long long)a.Nx * a.Ny < 0xffffffffLL - (1 << 20) ? rows_per_pass(a) : 0;
+    if (per) {
         switch (a.L) {
         case 8: return launch_rows<8>(a, per, num_sms, s);
         case 16: return launch_rows<16>(a, per, num_sms, s);
