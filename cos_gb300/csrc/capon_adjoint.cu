@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(32 * kAdjWarps) adjoint_kernel(AdjDev a)
 // (398 -> 335 us together with the gradient rows leaving as vector reductions
 // instead of a load and a store).  What bounds it: the FP32 pipe over the useful
 // lanes (30 of 32 at M=64, L=32, K=2), issue 58 %.  Gradients at [128][1024][64],
-// L=32, K=2: 335 us, 625 us as tiles.
+// L=32, K=2: 333 us, 625 us as tiles.
 static constexpr int kRowWarps = 8;
 
 struct AdjRowSmem {
@@ -179,9 +179,11 @@ COS_DEV void async_copy8(void *dst, const void *src, bool is)
 // `per` window rows at a time (at most 32, a lane each): a longer window, or one whose
 // accumulators leave fewer than two CTAs an SM, takes several passes over the rows, whose
 // gradients add up (backward pass at M=128, L=32, K=4, [64][520]: 840 -> 640 us; M=33, L=16,
-// K=17: 444 -> 354 us, both against register-blocked tiles).  A row none of whose pixels
-// has a gradient is not staged: the gradients are read two rows ahead.
-template <int L, int SB>
+// K=17: 444 -> 354 us, both against register-blocked tiles); SINGLE: one is enough, which
+// keeps the passes' bounds out of the rows' loop (333 us, 342 without it, in the case
+// above).  A row none of whose pixels has a gradient is not staged: the gradients are
+// read two rows ahead.
+template <int L, int SB, bool SINGLE>
 __global__ void __launch_bounds__(32 * kRowWarps, 2) adjoint_row_kernel(AdjDev a, int per)
 {
     static_assert(SB % 2 == 0 && L % 2 == 0, "channel pairs are 16 bytes");
@@ -197,7 +199,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 2) adjoint_row_kernel(AdjDev a
     // a warp's sum of g |w|^2.  Its terms cancel (gradients of either sign), so they are
     // added in FP64, one a row, and a CTA's sum goes out once
     __shared__ double dsum[kRowWarps];
-    if (lane == 0) dsum[warp] = 0.0;
+    double dacc = 0.0;
     for (int c = lane; c < M; c += 32) ths[c] = 0.f;
     for (int b = 0; b < 2; ++b) {   // the zero tails: samples past M, weights of the lanes without an item
         for (int c = M + lane; c < S.xs; c += 32) ((float2 *)mine)[b * S.xs + c] = make_float2(0.f, 0.f);
@@ -206,8 +208,8 @@ __global__ void __launch_bounds__(32 * kRowWarps, 2) adjoint_row_kernel(AdjDev a
     }
     const unsigned rows = (unsigned)a.Nx * a.Ny, step = gridDim.x * kRowWarps;
 #pragma unroll 1
-    for (int t0 = 0; t0 < 2 * a.K + 1; t0 += per) {
-        const int T = min(per, 2 * a.K + 1 - t0), items = T * nsb;   // window rows t0 .. t0+T-1
+    for (int t0 = 0; t0 < (SINGLE ? 1 : 2 * a.K + 1); t0 += per) {
+        const int T = SINGLE ? per : min(per, 2 * a.K + 1 - t0), items = T * nsb;   // window rows t0 .. t0+T-1
         // gradient of pixel y-t0-t on lane t; 0 where there is none
         auto grad = [&](unsigned row) {
             const unsigned bx = row / (unsigned)a.Ny;
@@ -268,7 +270,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 2) adjoint_row_kernel(AdjDev a
                     float wn = 0.f;
 #pragma unroll
                     for (int l = 0; l < L; ++l) wn += cabs2(w[l]);
-                    if (it == 0) dsum[warp] += (double)(g * wn);   // lane 0's
+                    if (it == 0) dacc += (double)(g * wn);
                 }
                 // e_s, s = s0 .. s0+SB-1: (re, im) parts as pair sums
                 float2 er[SB], ei[SB];
@@ -301,7 +303,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 2) adjoint_row_kernel(AdjDev a
                     er[j] = make_float2(re, -im);
                     ei[j] = make_float2(im, re);
                 }
-                float2 *const at = acc + min(t, T) * S.as + s0;   // lanes without an item: past the last
+                float2 *const at = acc + (SINGLE ? t : min(t, T)) * S.as + s0;   // lanes without an item: past the last
 #pragma unroll
                 for (int i = 0; i < SB + L - 1; i += 2) {
                     float2 G[2];
@@ -336,6 +338,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 2) adjoint_row_kernel(AdjDev a
             }
         }
     }
+    if (lane == 0) dsum[warp] = dacc;
     __syncthreads();
     if (a.gd && threadIdx.x == 0) {
         double v = 0.0;
@@ -393,10 +396,11 @@ static int launch_rows(const AdjDev &a, int per, int num_sms, cudaStream_t s)
         if (cost(sb) < cost(best)) best = sb;
     const size_t smem = AdjRowSmem(a.M, L, per, best).total;
     auto go = [&](auto kern) { return launch_adjoint_with(kern, a, units, smem, num_sms, s, per); };
-    return best == 2   ? go(adjoint_row_kernel<L, 2>)
-           : best == 4 ? go(adjoint_row_kernel<L, 4>)
-           : best == 6 ? go(adjoint_row_kernel<L, 6>)
-                       : go(adjoint_row_kernel<L, 8>);
+    const bool single = per == 2 * a.K + 1;
+    return best == 2   ? single ? go(adjoint_row_kernel<L, 2, true>) : go(adjoint_row_kernel<L, 2, false>)
+           : best == 4 ? single ? go(adjoint_row_kernel<L, 4, true>) : go(adjoint_row_kernel<L, 4, false>)
+           : best == 6 ? single ? go(adjoint_row_kernel<L, 6, true>) : go(adjoint_row_kernel<L, 6, false>)
+                       : single ? go(adjoint_row_kernel<L, 8, true>) : go(adjoint_row_kernel<L, 8, false>);
 }
 
 int launch_adjoint(const AdjDev &a, int num_sms, cudaStream_t s)
