@@ -28,11 +28,11 @@
 // same all along a diagonal and add up in P: 1.2 to 1.45 times as far from 64 bits for
 // K = 2 to 12, R itself 1.1 to 3.5 times.)
 // What bounds it: the FMA pipe, about 57 k packed operations a pixel at M=64, L=32,
-// K=2 with forward-backward averaging, at 50 to 65 % of its rate with waits at the
-// barriers between the phases; what fits of the row sums into shared memory gives the
-// threads of a phase.  Measured, 60 k pixels at M=48, L=24, K=2 with weights: 1.44 ms in
-// the precise pipeline, 0.21 ms here + 0.13 ms in the solve stage; 65 k pixels at M=64,
-// L=32, K=2 with forward-backward averaging: 2.56 ms, 0.38 + 0.17 ms.
+// K=2 with forward-backward averaging, at 50 to 65 % of its rate (issue 49 %, L1 59 %),
+// with waits at the barriers between the phases; what fits of the row sums into shared
+// memory gives the threads of a phase.  Measured, 60 k pixels at M=48, L=24, K=2 with
+// weights: 1.44 ms in the precise pipeline, 0.21 ms here + 0.15 ms in the solve stage; 65 k
+// pixels at M=64, L=32, K=2 with forward-backward averaging: 2.56 ms, 0.38 + 0.20 ms.
 #include <algorithm>
 #include <cmath>
 

@@ -13,7 +13,7 @@
 // along, a row scaled by its pivot's inverse square root and broadcast through shared
 // memory; a product is formed and then subtracted.  The fused kernels' form, R =
 // L D L^H with the product subtracted by two fmas, is faster (65 k pixels, L = 32, z
-// and P: 0.17 ms, 0.19 so; 60 k pixels, L = 24, weights: 0.13 and 0.15) but rounds
+// and P: 0.17 ms, 0.20 so; 60 k pixels, L = 24, weights: 0.12 and 0.15) but rounds
 // twice at the entry's size, and its update carries the rounding of the multipliers,
 // which a factor used on both sides does not: w was 1.1 to 1.27 times as far from 64
 // bits as in the precise pipeline at L = 33 to 64 (P up to 1.19 times), 0.95 to 1.01

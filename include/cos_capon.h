@@ -93,8 +93,8 @@ typedef struct cos_capon_opts {
     int fb;         /* 1: forward-backward averaged covariance (R + J R^T J)/2
                        before loading and any beamspace transform
                        (getCaponAllC.pyx:346-347, getCaponPy_ref.py:103-104);
-                       element space runs the float-float pipeline, beamspace
-                       supports Nb <= 5                                        */
+                       element space runs the general path (the float-float
+                       pipeline with refinement), beamspace supports Nb <= 5    */
     int segment;    /* COS_CAPON_FORM_SLIDING_INVERSE: pixels along range per
                        fresh build-up of the inverse; 0 = 8                    */
 } cos_capon_opts;
