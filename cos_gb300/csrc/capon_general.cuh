@@ -9,15 +9,18 @@
 // factorisations, since a warp's triangle leaves no room to load ahead.
 //
 // G lanes own one pixel, lane r the columns j = m*G + r of the upper triangle
-// (m < LP/G).  R = U^H U (matrixDecompc.pyx:19-50), the right-hand sides carried
-// along, a row scaled by its pivot's inverse square root and broadcast through shared
-// memory; a product is formed and then subtracted.  The fused kernels' form, R =
-// L D L^H with the product subtracted by two fmas, is faster (65 k pixels, L = 32, z
-// and P: 0.17 ms, 0.20 so; 60 k pixels, L = 24, weights: 0.12 and 0.15) but rounds
-// twice at the entry's size, and its update carries the rounding of the multipliers,
-// which a factor used on both sides does not: w was 1.1 to 1.27 times as far from 64
-// bits as in the precise pipeline at L = 33 to 64 (P up to 1.19 times), 0.95 to 1.01
-// times so.  A subarray length between two
+// (m < LP/G), the right-hand sides carried along, a pivot row broadcast through
+// shared memory.  Two factorisations (matrixDecompc.pyx:19-50), by the subarray length:
+//   LP <= 16  that of the fused kernels, R = L D L^H: rows broadcast as they are and
+//             scaled by their readers, a product subtracted by two fmas;
+//   above     R = U^H U: rows scaled by the pivot's inverse square root before they
+//             are broadcast, a product formed and then subtracted.
+// The first is faster (65 k pixels, L = 32, z and P: 0.17 ms, 0.20 by the second; 60 k
+// pixels, L = 24, weights: 0.12 and 0.15), but rounds twice at the entry's size, and its
+// update carries the rounding of the multipliers, which a factor used on both sides
+// does not.  Against 64 bits, as a multiple of the precise pipeline's error: w 0.80,
+// 0.94, 1.03, 1.04, 1.10, 1.16, 1.27 at L = 5, 16, 20, 24, 32, 40, 64 by the first, 0.92,
+// 0.95, 0.99, 0.99, 0.99, 1.01, 1.01 by the second, P alike.  A subarray length between two
 // instantiations is padded in front: rows and columns 0 .. pad-1 (pad = LP - L)
 // are an identity with zero right-hand sides, and the unrolled steps of those
 // rows are skipped, so that padding costs idle column slots only -- the steps
@@ -52,6 +55,7 @@ struct SolveCfg {
     static constexpr int LP = LP_, G = G_, MAXPAD = MAXPAD_;  // pad < MAXPAD
     static constexpr int WARPS = WARPS_, BLOCKS = BLOCKS_;
     static constexpr int NM = LP / G, PPW = 32 / G;
+    static constexpr bool LDL = LP <= 16;   // R = L D L^H, else U^H U
     // float4 slots of a pixel's shared area: two pivot rows, or the exchange
     // area of the back substitution
     static constexpr int RB = 2 * (LP + 1), XCH = (G * (G + 1) + 1) / 2;
@@ -139,26 +143,29 @@ solve_kernel(FrameDev f, const float2 *__restrict__ work, long long npix, unsign
         bool bad = false;
         float s11 = 0.f, s11l = 0.f;  // high part and the sum of its rounding errors
         float2 s12 = make_float2(0.f, 0.f);
-        // row `row` and its right-hand sides by the pivot's inverse square root, then
-        // the row as (-Re, +Im, -Im, -Re) of U[row][j]; slot LP carries the right-hand sides
+        // row `row` as (-Re, +Im, -Im, -Re) of A[row][j]; slot LP carries the row's
+        // right-hand sides.  U^H U: all of them by the pivot's inverse square root first
         auto publish = [&](auto rc, float4 *buf) __attribute__((always_inline)) {
             constexpr int row = decltype(rc)::value, mrow = row / G;
-            const float dv = __shfl_sync(0xffffffffu, A[row][mrow].x, row % G, G);
-            bad |= !(dv > 0.f);
-            // the unit's approximation and one Newton step: its error is common to the
-            // whole row
-            const float y0 = rsqrtf(dv), inv = fmaf(0.5f * y0, fmaf(-dv * y0, y0, 1.f), y0);
+            if constexpr (!C::LDL) {
+                const float dv = __shfl_sync(0xffffffffu, A[row][mrow].x, row % G, G);
+                bad |= !(dv > 0.f);
+                // the unit's approximation and one Newton step: its error is common to the
+                // whole row
+                const float y0 = rsqrtf(dv), inv = fmaf(0.5f * y0, fmaf(-dv * y0, y0, 1.f), y0);
 #pragma unroll
-            for (int m = mrow; m < NM; ++m) {
-                A[row][m] = cscale(A[row][m], inv);
+                for (int m = mrow; m < NM; ++m) A[row][m] = cscale(A[row][m], inv);
+                if (r == row % G) {
+                    if (W) dinv[mrow] = inv;
+                    b1[mrow] = cscale(b1[mrow], inv);
+                    if (!W) b2[mrow] = cscale(b2[mrow], inv);
+                }
+            }
+#pragma unroll
+            for (int m = mrow; m < NM; ++m)
                 buf[m * G + r] = make_float4(-A[row][m].x, A[row][m].y, -A[row][m].y, -A[row][m].x);
-            }
-            if (r == row % G) {
-                if (W) dinv[mrow] = inv;
-                b1[mrow] = cscale(b1[mrow], inv);
-                if (!W) b2[mrow] = cscale(b2[mrow], inv);
+            if (r == row % G)
                 buf[LP] = make_float4(b1[mrow].x, b1[mrow].y, W ? 0.f : b2[mrow].x, W ? 0.f : b2[mrow].y);
-            }
         };
         __syncwarp();  // the area's readers of the last pixel are done
         if (pad == 0) publish(std::integral_constant<int, 0>{}, rb);
@@ -175,28 +182,42 @@ solve_kernel(FrameDev f, const float2 *__restrict__ work, long long npix, unsign
                 float4 *const rbi = rb + (i & 1) * (LP + 1);
                 __syncwarp();
                 const float4 yy = rbi[LP];
-                const float2 y1 = make_float2(yy.x, yy.y), y2 = make_float2(yy.z, yy.w);
+                // rdv scales the row and its right-hand sides at the reader (L D L^H)
+                float rdv = 1.f;
+                if constexpr (C::LDL) {
+                    const float dv = -rbi[i].x;
+                    bad |= !(dv > 0.f);
+                    rdv = __frcp_rn(dv);
+                    if (W && r == oi) dinv[mi] = rdv;
+                }
+                auto scaled = [&](float v) { return C::LDL ? v * rdv : v; };
+                const float2 y1 = make_float2(scaled(yy.x), scaled(yy.y)), y2 = make_float2(scaled(yy.z), scaled(yy.w));
                 {
-                    const float t = cabs2(y1), s = s11 + t;
+                    const float t = fmaf(yy.x, y1.x, yy.y * y1.y), s = s11 + t;
                     s11l += t - (s - s11);
                     s11 = s;
                 }
-                if (!W) s12 = cadd(s12, cconjmul(y1, y2));
+                if (!W) s12 = cadd(s12, cconjmul(make_float2(yy.x, yy.y), y2));
                 const float2 y1s = make_float2(y1.y, y1.x), y2s = make_float2(y2.y, y2.x);
+                // c + b d + a e, the sum of products first or two fmas
+                auto update = [&](float2 a, float2 e, float2 b, float2 d, float2 c) __attribute__((always_inline)) {
+                    return C::LDL ? ffma2(a, e, ffma2(b, d, c)) : fadd2(c, ffma2(a, e, ffma2(b, d, zero)));
+                };
                 float2 vrr[NM], vii[NM];
 #pragma unroll
                 for (int m = mi; m < NM; ++m) {
                     const float2 v = A[i][m];
                     const float2 n1 = make_float2(-v.x, -v.x), n2 = make_float2(-v.y, v.y);
-                    const float2 t1 = fadd2(b1[m], ffma2(n2, y1s, ffma2(n1, y1, zero)));
+                    const float2 t1 = update(n2, y1s, n1, y1, b1[m]);
                     const bool below = m > mi || r > oi;
                     if (below) b1[m] = t1;
                     if (!W) {
-                        const float2 t2 = fadd2(b2[m], ffma2(n2, y2s, ffma2(n1, y2, zero)));
+                        const float2 t2 = update(n2, y2s, n1, y2, b2[m]);
                         if (below) b2[m] = t2;
                     }
-                    vrr[m] = make_float2(v.x, v.x);
-                    vii[m] = make_float2(v.y, v.y);
+                    const float vr = scaled(v.x), vi = scaled(v.y);
+                    vrr[m] = make_float2(vr, vr);
+                    vii[m] = make_float2(vi, vi);
                 }
                 // row i+1 first, published before the bulk of the update
 #pragma unroll
@@ -205,8 +226,7 @@ solve_kernel(FrameDev f, const float2 *__restrict__ work, long long npix, unsign
 #pragma unroll
                     for (int m = mi; m < NM; ++m)
                         if (m >= k / G)
-                            A[k][m] = fadd2(A[k][m], ffma2(vii[m], make_float2(u4.z, u4.w),
-                                                           ffma2(vrr[m], make_float2(u4.x, u4.y), zero)));
+                            A[k][m] = update(vii[m], make_float2(u4.z, u4.w), vrr[m], make_float2(u4.x, u4.y), A[k][m]);
                     if constexpr (i + 1 < LP)
                         if (k == i + 1) publish(std::integral_constant<int, i + 1>{}, nxt);
                 }
@@ -221,7 +241,7 @@ solve_kernel(FrameDev f, const float2 *__restrict__ work, long long npix, unsign
             if (bad) atomicOr(status, ERR_NOT_PD);
         }
         if constexpr (W) {
-            // U x = b1 by blocks of G rows, last block first, through the
+            // (D L^H) x = b1, or U x = b1, by blocks of G rows, last block first, through the
             // exchange area (the fused w mode's scheme, capon_fused.cuh)
             float2 xv[NM];
 #pragma unroll
