@@ -24,7 +24,8 @@ def exact_R(x, L, K, fb, d):
 
 # Nx, pixels, M, L, K
 CASES = [(2, 9, 5, 1, 1), (2, 5, 7, 2, 0), (2, 70, 17, 8, 1), (2, 13, 33, 17, 2), (3, 40, 48, 24, 3), (2, 11, 62, 31, 4),
-         (1, 6, 72, 24, 12), (1, 9, 24, 12, 60), (1, 7, 80, 40, 2), (1, 5, 126, 63, 1), (1, 4, 300, 20, 2), (1, 3, 63, 63, 2)]
+         (1, 6, 72, 24, 12), (1, 9, 24, 12, 60), (1, 7, 80, 40, 2), (1, 5, 126, 63, 1), (1, 4, 300, 20, 2), (1, 3, 63, 63, 2),
+         (30, 150, 48, 24, 2), (1, 8, 126, 63, 16)]
 
 
 @pytest.mark.parametrize("fb", [0, 1])
